@@ -60,6 +60,9 @@ struct GridCtx {
   DevVec<float> satw_t;
   DevVec<int> sati_t;
   DevVec<float> cumulw_t;
+  DevVec<float> cumt;               ///< CUMULW by (IK2, IK, J - ITH), where it is a function of those
+  bool has_cumt = false;
+  int nsat_eff = -1;                ///< SATWEIGHTS rows to sum
   St4Dev host{};                    ///< the kernel parameters (module state of the commit)
   St4Dev* dev = nullptr;            ///< their device copy
   ~GridCtx() {
@@ -91,7 +94,8 @@ void refresh(GridCtx& g) {
                    g.f[st4::A_ECOS].ptr,  g.f[st4::A_TH].ptr,    g.satw_t.ptr,
                    g.cumulw_t.ptr, g.f[st4::A_DCKI].ptr, g.f[st4::A_QBI].ptr,
                    m.f[st4::A_TAUT].ptr,  m.f[st4::A_TAUHFT].ptr, m.f[st4::A_TAUHFT2].ptr,
-                   m.f[st4::A_FWTABLE].ptr, g.sati_t.ptr,         g.i[st4::A_IKTAB].ptr};
+                   m.f[st4::A_FWTABLE].ptr, g.sati_t.ptr,         g.i[st4::A_IKTAB].ptr,
+                   g.has_cumt ? g.cumt.ptr : nullptr, g.nsat_eff};
   (void)a;
   g.host.p = st4::current_params(g.reg, m.reg);
   g.host.f = st4::make_fields(g.reg, q);
@@ -438,6 +442,10 @@ int ww_st4_commit(int igrid) {
     std::vector<float> ct;
     st4::transpose_cumulw(g.reg, ct);
     g.cumulw_t.upload(ct);
+    const std::vector<float> cumt = st4::toeplitz_cumulw(g.reg);
+    g.has_cumt = !cumt.empty();
+    g.cumt.upload(cumt);
+    g.nsat_eff = st4::sat_rows(g.reg);
     g.f[st4::A_CUMULW].upload({});  // only the transposed copy is read
     refresh(g);
     g.ready = true;

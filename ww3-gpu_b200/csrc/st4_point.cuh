@@ -105,6 +105,10 @@ struct Fields {
   int nsat, sat_ld;
   const float* cumulw;  ///< CUMULW transposed: CUMULW(i,j) = cumulw[(j-1) + (i-1)*cumulw_ld]
   int cumulw_ld;
+  /// CUMULW as a function of (IK2, IK, J - ITH), where the registered table is one: CUMULW((IK2-1)
+  /// NTH + J, (IK-1) NTH + ITH) = cumt[((IK2-1) NK + IK-1) (2 NTH - 1) + J - ITH + NTH - 1]; else null.
+  const float* cumt;
+  int nsat_eff;  ///< SATWEIGHTS rows up to the last that is not zero for the same bin as those after it
   const float *dcki, *qbi;  ///< (NKHS, NKD)
   const int* iktab;         ///< IKTAB(ik,id) = iktab[(ik-1) + (id-1)*iktab_ld]
   int iktab_ld;

@@ -10,6 +10,7 @@
 // registrations accepted), :472-584 (init, set, commit status codes).
 #pragma once
 
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -150,12 +151,52 @@ inline void transpose_cumulw(const GridReg& g, std::vector<float>& t) {
     for (size_t i = 0; i < n; ++i) t[j + i * n] = c.f[i + j * n];
 }
 
+/// CUMULW by (IK2, IK, J - ITH) (pt::Fields::cumt), or an empty vector when the registered table is
+/// not a function of those (INSIN4's is: its angle is TH(J) - TH(ITH)); 374 KB instead of 6.7 MB at 36x36.
+inline std::vector<float> toeplitz_cumulw(const GridReg& g) {
+  const Reg& c = g.a[A_CUMULW];
+  const int nk = g.p.nk, nth = g.p.nth, ld = 2 * nth - 1;
+  const size_t n = c.ext[0];
+  std::vector<float> t(static_cast<size_t>(nk) * nk * ld, 0.0f);
+  for (int ik = 0; ik < nk; ++ik)
+    for (int ik2 = 0; ik2 < nk; ++ik2) {
+      float* const row = t.data() + (static_cast<size_t>(ik2) * nk + ik) * ld + nth - 1;
+      for (int ith = 0; ith < nth; ++ith) {
+        const float* const col =
+            c.f.data() + static_cast<size_t>(ik2) * nth + (static_cast<size_t>(ik) * nth + ith) * n;
+        for (int j = 0; j < nth; ++j) {
+          if (ith == 0 || j == 0) row[j - ith] = col[j];  // the first value of each J - ITH
+          else if (std::memcmp(&row[j - ith], &col[j], sizeof(float)) != 0) return {};
+        }
+      }
+    }
+  return t;
+}
+
+/// SATWEIGHTS rows to sum: from the returned row on, every row is zero with the same SATINDICES as
+/// that row (pt::Fields::nsat_eff).
+inline int sat_rows(const GridReg& g) {
+  const Reg& w = g.a[A_SATWEIGHTS];
+  const Reg& x = g.a[A_SATINDICES];
+  const int nsat = w.ext[0], mth = w.ext[1];
+  int n = nsat;
+  for (; n > 0; --n) {
+    for (int ith = 0; ith < mth; ++ith) {
+      const size_t o = static_cast<size_t>(ith) * nsat;
+      if (w.f[o + n - 1] != 0.0f || (n < nsat && x.i[o + n - 1] != x.i[o + n])) return n;
+    }
+  }
+  return n;
+}
+
 /// Fields over host-resident copies (the CPU build of the kernels) or over device copies whose
 /// pointers the caller fills in the same order (abi_st4.cpp).
 struct FieldPtrs {
   const float *sig, *sig2, *dsip, *dden, *dden2, *esin, *ecos, *th, *satw_t, *cumulw_t, *dcki,
       *qbi, *taut, *tauhft, *tauhft2, *fwtable;
   const int *sati_t, *iktab;
+  const float* cumt = nullptr;
+  int nsat_eff = -1;  ///< sat_rows of the registration the pointers belong to (-1: every row)
 };
 
 inline pt::Fields make_fields(const GridReg& g, const FieldPtrs& q) {
@@ -174,6 +215,8 @@ inline pt::Fields make_fields(const GridReg& g, const FieldPtrs& q) {
   f.sat_ld = g.a[A_SATWEIGHTS].ext[1];
   f.cumulw = q.cumulw_t;
   f.cumulw_ld = g.a[A_CUMULW].ext[0];
+  f.cumt = q.cumt;
+  f.nsat_eff = q.nsat_eff < 0 ? f.nsat : q.nsat_eff;
   f.dcki = q.dcki;
   f.qbi = q.qbi;
   f.iktab = q.iktab;

@@ -36,11 +36,10 @@ struct SrceStep {
 /// Threads of every ST4 CTA (one CTA per point).
 constexpr int kSt4Block = 256;
 
-/// Threads of a W3SRCE CTA, and the CTAs per SM it is built for: one point's serial chains
-/// leave most of its warps waiting at barriers, so more points per SM (their shared part fits
-/// four times, their registers four times 128 threads) beat more threads per point.
-constexpr int kSrceBlock = pt::kSrceSplit ? 128 : 256;
-constexpr int kSrceMinBlocks = pt::kSrceSplit ? 4 : 2;
+/// Threads of a W3SRCE CTA, and the CTAs per SM it is built for: one CTA's ordered chains run beside
+/// the other's parallel phases.
+constexpr int kSrceBlock = 384;
+constexpr int kSrceMinBlocks = 2;
 
 /// One grid's W3SRCE work buffers: the work queue's counter and the global part of the resident
 /// CTAs' working sets (grow-only; it stays in L2 at these sizes). Owned by the grid's context.
@@ -110,9 +109,6 @@ int srce_max_ctas_per_sm(const pt::SrceLayout& L);
 /// Limits the W3SRCE kernels to `ctas` CTAs per SM (0: all that fit) with the shared-memory
 /// carveout they need, the rest of the SM's memory left to L1 (the autotuner's choice).
 void srce_set_ctas_per_sm(const pt::SrceLayout& L, int ctas);
-
-/// CTAs of a W3SRCE launch on npts points of these tables (the resident grid, at most npts).
-int srce_resident_ctas(const pt::SrceLayout& L, int npts);
 
 /// Allocates launch_srce_multi's work buffers for `total` points of layout L (synchronous).
 void srce_multi_reserve(const pt::SrceLayout& L, int total, SrceWork& work);

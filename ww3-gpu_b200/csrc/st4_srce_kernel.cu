@@ -1,12 +1,10 @@
 // ww3-gpu_b200/csrc/st4_srce_kernel.cu
-// The ST4 source terms and W3SRCE on sm_100a: one CTA of 256 threads per sea point, the point's
-// working set in shared memory, the phases of st4_point.cuh / srce_point.cuh.
+// The ST4 source terms (one CTA per sea point, the phases of st4_point.cuh) and W3SRCE (up to
+// pt::kSlots points per CTA, srce_point.cuh) on sm_100a.
 //
-// W3SRCE runs on a persistent grid: each CTA takes the next point from a global counter as it
-// finishes one, so the uneven number of substeps per point (the dynamic integration stops when
+// W3SRCE runs on a persistent grid: a CTA takes the next point from a global counter as one of its
+// slots finishes one, so the uneven number of substeps per point (the dynamic integration stops when
 // the point's DTTOT reaches DTG) balances across the SMs instead of leaving a tail of idle CTAs.
-// The scalar state of a point sits in static shared memory, its spectra and work arrays in
-// dynamic shared memory (about 100 KiB at 36x36, two CTAs per SM).
 #include "st4_srce.cuh"
 
 #include "wwb_common.hpp"
@@ -84,138 +82,256 @@ __global__ void __launch_bounds__(kSt4Block) spr4_kernel(
   }
 }
 
-/// One sea point of a W3SRCE batch by the whole CTA: its spectrum (VA column jsea[n], or row n)
-/// and packets into the working set, srce_point, and back. w is the CTA's dynamic shared
-/// memory, gw its slice of the global scratch.
-__device__ __forceinline__ void srce_one(const SrceDev* __restrict__ d, const SrceStep& step,
-                                         int n, float* spec, const int* jsea, const float* wn1,
-                                         const float* cg1, const float* pin, float* psc,
-                                         float* whitecap, float* taubbl, float* tauice,
-                                         int* shave, float* w, float* gw, pt::SrceSh& sh) {
-  const pt::SrceLayout& L = d->L;
-  const int ns = L.nspec, nk = L.nk;
-  const pt::Cta cta{static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x)};
-  float* const sp = spec + (jsea ? static_cast<size_t>(jsea[n]) : static_cast<size_t>(n)) * ns;
-  for (int i = threadIdx.x; i < ns; i += blockDim.x) w[L.spec + i] = sp[i];
-  for (int i = threadIdx.x; i < nk; i += blockDim.x) {
-    w[L.wn1 + i] = wn1[static_cast<size_t>(n) * nk + i];
-    w[L.cg1 + i] = cg1[static_cast<size_t>(n) * nk + i];
-  }
-  if (threadIdx.x == 0)
-    pt::srce_psc_in(sh, psc + static_cast<size_t>(n) * srce::NPSC,
-                    whitecap + 4 * static_cast<size_t>(n), taubbl + 2 * static_cast<size_t>(n),
-                    tauice + 2 * static_cast<size_t>(n));
-  __syncthreads();
-  const pt::SrceCtx x{&d->p, &d->g, &d->q, &d->f, &d->n,
-                      pt::srce_in(step.it, step.inflags24, step.flogrd57, step.flogrd58, step.dtg,
-                                  pin + static_cast<size_t>(n) * srce::NPIN),
-                      w, gw, &L, &sh};
-  pt::srce_point(cta, x);
-  for (int i = threadIdx.x; i < ns; i += blockDim.x) sp[i] = w[L.spec + i];
-  if (threadIdx.x == 0)
-    pt::srce_psc_out(sh, psc + static_cast<size_t>(n) * srce::NPSC,
-                     whitecap + 4 * static_cast<size_t>(n), taubbl + 2 * static_cast<size_t>(n),
-                     tauice + 2 * static_cast<size_t>(n), shave + n);
-  __syncthreads();
-}
+/// What the CTA's threads agree on: the job whose points it integrates, the slots' points, and a queue
+/// entry taken but not yet loaded (it belongs to another job when `foreign`).
+struct SrceCtl {
+  SrceJob job;
+  int pt[pt::kSlots];
+  int pending, foreign, empty;
+  unsigned fresh;
+};
 
-__global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
-    const SrceDev* __restrict__ d, SrceStep step, int npts, float* spec, const int* jsea,
-    const float* wn1, const float* cg1, const float* pin, float* psc, float* whitecap,
-    float* taubbl, float* tauice, int* shave, int* counter, float* scratch) {
-  extern __shared__ __align__(16) float w[];
-  __shared__ pt::SrceSh sh;
-  __shared__ int cur;
-  float* const gw = scratch + static_cast<size_t>(blockIdx.x) * static_cast<size_t>(d->L.total_g);
-  for (;;) {
-    if (threadIdx.x == 0) cur = atomicAdd(counter, 1);
-    __syncthreads();
-    const int n = cur;
-    if (n >= npts) break;
-    srce_one(d, step, n, spec, jsea, wn1, cg1, pin, psc, whitecap, taubbl, tauice, shave, w, gw,
-             sh);
-  }
-}
+/// Points of one job from the launch's work queue.
+struct QueuePoints {
+  SrceCtl& ctl;
+  int total;
+  int* counter;
 
-/// W3SRCE over the points of several grids in one persistent launch: one work queue over
-/// (grid, point), the job of queue entry q the last one whose first entry is <= q. Every job has
-/// the same working-set layout (checked on the host), so one CTA takes any grid's points.
-__global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
-    const SrceJob* __restrict__ jobs, int njobs, int total, int* counter, float* scratch) {
-  extern __shared__ __align__(16) float w[];
-  __shared__ pt::SrceSh sh;
-  __shared__ int cur;
-  float* const gw =
-      scratch + static_cast<size_t>(blockIdx.x) * static_cast<size_t>(jobs[0].d->L.total_g);
-  for (;;) {
-    if (threadIdx.x == 0) cur = atomicAdd(counter, 1);
-    __syncthreads();
-    const int q = cur;
-    if (q >= total) break;
-    int lo = 0, hi = njobs - 1;  // the job holding q: first[lo] <= q < first[lo + 1]
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (jobs[mid].first <= q) lo = mid;
-      else hi = mid - 1;
+  __device__ __forceinline__ void load(const pt::Grp& c, const pt::SrceGroup& x,
+                                       pt::SlotList& fresh) {
+    const pt::SrceLayout& L = *x.L;
+    if (ctl.empty || ctl.foreign) return;
+    bool room = false;
+    for (int k = 0; k < x.ns; ++k) room = room || x.sh[k].state == pt::kIdle;
+    if (!room) return;
+    __syncthreads();  // every thread has read the states and the queue's
+    if (c.tid == 0) {
+      unsigned m = 0;
+      for (int k = 0; k < x.ns; ++k) {
+        if (x.sh[k].state != pt::kIdle) continue;
+        const int q = ctl.pending >= 0 ? ctl.pending : atomicAdd(counter, 1);
+        ctl.pending = -1;
+        if (q >= total) {
+          ctl.empty = 1;
+          break;
+        }
+        if (q < ctl.job.first || q >= ctl.job.first + ctl.job.npts) {
+          ctl.pending = q;
+          ctl.foreign = 1;
+          break;
+        }
+        ctl.pt[k] = q - ctl.job.first;
+        x.sh[k].state = ctl.job.step.it != 0 ? pt::kFresh1 : pt::kFresh2;
+        m |= 1u << k;
+      }
+      ctl.fresh = m;
     }
-    const SrceJob& j = jobs[lo];
-    srce_one(j.d, j.step, q - j.first, j.spec, j.jsea, j.wn1, j.cg1, j.pin, j.psc, j.whitecap,
-             j.taubbl, j.tauice, j.shave, w, gw, sh);
+    __syncthreads();
+    const unsigned m = ctl.fresh;
+    for (int k = 0; k < x.ns; ++k)
+      if (m >> k & 1) fresh.add(k);
+    if (fresh.n == 0) return;
+    const SrceJob& j = ctl.job;
+    pt::each_bin(c, fresh, L.nspec, [&](int k, int i) {
+      const int n = ctl.pt[k];
+      const size_t col = j.jsea ? static_cast<size_t>(j.jsea[n]) : static_cast<size_t>(n);
+      x.s(k, L.spec)[i] = j.spec[col * L.nspec + i];
+    });
+    pt::each_row(c, fresh, L.nk, [&](int k, int ik) {
+      const size_t o = static_cast<size_t>(ctl.pt[k]) * L.nk + ik;
+      x.s(k, L.wn1)[ik] = j.wn1[o];
+      x.s(k, L.cg1)[ik] = j.cg1[o];
+    });
+    pt::each_chain(c, 0, fresh, [&](int k) {
+      const size_t n = ctl.pt[k];
+      pt::SrceSh& s = x.sh[k];
+      pt::srce_psc_in(s, j.psc + n * srce::NPSC, j.whitecap + 4 * n, j.taubbl + 2 * n,
+                      j.tauice + 2 * n);
+      s.r.z0 = s.r.cd = s.r.emean = s.r.fmean = s.r.fmean1 = s.r.amax = s.r.fmeanws = 0.0f;
+      s.in = pt::srce_in(j.step.it, j.step.inflags24, j.step.flogrd57, j.step.flogrd58, j.step.dtg,
+                         j.pin + n * srce::NPIN);
+    });
+    __syncthreads();
+  }
+
+  __device__ __forceinline__ void store(const pt::Grp& c, const pt::SrceGroup& x,
+                                        const pt::SlotList& done) {
+    const pt::SrceLayout& L = *x.L;
+    const SrceJob& j = ctl.job;
+    pt::each_bin(c, done, L.nspec, [&](int k, int i) {
+      const int n = ctl.pt[k];
+      const size_t col = j.jsea ? static_cast<size_t>(j.jsea[n]) : static_cast<size_t>(n);
+      j.spec[col * L.nspec + i] = x.s(k, L.spec)[i];
+    });
+    pt::each_chain(c, 0, done, [&](int k) {
+      const size_t n = ctl.pt[k];
+      pt::srce_psc_out(x.sh[k], j.psc + n * srce::NPSC, j.whitecap + 4 * n, j.taubbl + 2 * n,
+                       j.tauice + 2 * n, j.shave + n);
+      x.sh[k].state = pt::kIdle;
+    });
+    __syncthreads();
+  }
+};
+
+/// W3SRCE over the points of one or several grids in one persistent launch: one work queue over
+/// (grid, point), the job of queue entry q the last one whose first entry is <= q. A CTA integrates up
+/// to ns points of one job at a time (srce_point.cuh) and turns to the next job when its slots are
+/// empty. Every job has the same working-set layout (checked on the host).
+__global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
+    SrceJob one, const SrceJob* __restrict__ jobs, int njobs, int total, int ns, int* counter,
+    float* scratch) {
+  extern __shared__ __align__(16) float w[];
+  __shared__ pt::SrceSh sh[pt::kSlots];
+  __shared__ SrceCtl ctl;
+  __shared__ SrceDev dev;
+  const pt::Grp c{static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x)};
+  if (threadIdx.x == 0) {
+    ctl.pending = -1;
+    for (int k = 0; k < pt::kSlots; ++k) sh[k].state = pt::kIdle;
+  }
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int q = ctl.pending >= 0 ? ctl.pending : atomicAdd(counter, 1);
+      ctl.pending = q;
+      ctl.foreign = 0;
+      ctl.empty = q >= total;
+      if (q < total) {
+        if (jobs == nullptr) {
+          ctl.job = one;
+        } else {
+          int lo = 0, hi = njobs - 1;  // the job holding q: first[lo] <= q < first[lo + 1]
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (jobs[mid].first <= q) lo = mid;
+            else hi = mid - 1;
+          }
+          ctl.job = jobs[lo];
+        }
+      }
+    }
+    __syncthreads();
+    if (ctl.empty) break;
+    {
+      const int* const from = reinterpret_cast<const int*>(ctl.job.d);
+      int* const to = reinterpret_cast<int*>(&dev);
+      for (int i = threadIdx.x; i < static_cast<int>(sizeof(SrceDev) / sizeof(int)); i += blockDim.x)
+        to[i] = from[i];
+    }
+    __syncthreads();
+    float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
+    const pt::SrceGroup x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
+                          w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns};
+    QueuePoints src{ctl, total, counter};
+    pt::srce_run(c, x, src);
   }
 }
 
-/// CTAs per SM of the W3SRCE kernels (0: all that fit), set by the autotuner.
+/// CTAs per SM of the W3SRCE kernel (0: all that fit), set by the autotuner.
 int g_srce_ctas_per_sm = 0;
 
-/// Resident CTAs per SM of a kernel at this shared memory, at least 1 (for the W3SRCE kernels,
-/// at most the autotuner's choice).
+/// Resident CTAs of an ST4 kernel at this shared memory, at most one per point.
 template <class K>
-int resident_grid(K k, size_t smem, int npts, int block = kSt4Block, bool srce = false) {
+int resident_grid(K k, size_t smem, int npts) {
   WWB_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
   int per_sm = 0;
-  WWB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block, smem));
-  if (per_sm < 1) throw CudaError(cudaErrorInvalidConfiguration, "st4/srce occupancy");
-  if (srce && g_srce_ctas_per_sm > 0 && g_srce_ctas_per_sm < per_sm)
-    per_sm = g_srce_ctas_per_sm;
+  WWB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kSt4Block, smem));
+  if (per_sm < 1) throw CudaError(cudaErrorInvalidConfiguration, "st4 occupancy");
   const long long resident = static_cast<long long>(per_sm) * runtime().sm_count;
   return static_cast<int>(npts < resident ? npts : resident);
+}
+
+/// Dynamic shared memory of a W3SRCE CTA with ns slots.
+size_t srce_smem(const pt::SrceLayout& L, int ns) {
+  return static_cast<size_t>(pt::srce_shared_floats(L, ns)) * sizeof(float);
+}
+constexpr size_t kSrceStatic =
+    sizeof(pt::SrceSh) * pt::kSlots + sizeof(SrceCtl) + sizeof(SrceDev) + 64;
+
+/// A W3SRCE launch: slots per CTA, CTAs, shared memory.
+struct SrcePlan {
+  int ns, grid;
+  size_t smem;
+};
+int srce_per_sm(const pt::SrceLayout& L, int ns) {
+  const size_t smem = srce_smem(L, ns);
+  WWB_CHECK(cudaFuncSetAttribute(srce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(smem)));
+  int per_sm = 0;
+  WWB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, srce_kernel, kSrceBlock, smem));
+  if (per_sm < 1) throw CudaError(cudaErrorInvalidConfiguration, "srce occupancy");
+  return g_srce_ctas_per_sm > 0 && g_srce_ctas_per_sm < per_sm ? g_srce_ctas_per_sm : per_sm;
+}
+/// Slots a CTA of this layout can have: all of them where as many CTAs fit an SM as with one.
+int srce_max_slots(const pt::SrceLayout& L) {
+  const size_t budget = 233472 / kSrceMinBlocks - 1024;
+  for (int ns = pt::kSlots; ns > 1; --ns)
+    if (srce_smem(L, ns) + kSrceStatic <= budget) return ns;
+  return 1;
+}
+/// One point per CTA until every SM has its CTAs, then more: a launch lasts as long as its longest
+/// point, and a point alone in its CTA is integrated fastest.
+SrcePlan srce_plan(const pt::SrceLayout& L, int npts) {
+  if (srce_smem_bytes(L) == 0)
+    throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
+  const int most = srce_max_slots(L), sms = runtime().sm_count;
+  for (int ns = 1;; ++ns) {
+    const long long ctas = static_cast<long long>(srce_per_sm(L, ns)) * sms;
+    if (ns == most || ctas * ns >= npts) {
+      const long long want = (static_cast<long long>(npts) + ns - 1) / ns;
+      return SrcePlan{ns, static_cast<int>(want < ctas ? want : ctas), srce_smem(L, ns)};
+    }
+  }
+}
+void srce_reserve_plan(const pt::SrceLayout& L, const SrcePlan& plan, SrceWork& work) {
+  const size_t need = static_cast<size_t>(plan.grid) * plan.ns * static_cast<size_t>(L.total_g);
+  if (work.counter == nullptr) WWB_CHECK(cudaMalloc(&work.counter, sizeof(int)));
+  if (need > work.scratch_n) {
+    if (work.scratch) WWB_CHECK(cudaFree(work.scratch));
+    work.scratch = nullptr;
+    work.scratch_n = 0;
+    WWB_CHECK(cudaMalloc(&work.scratch, need * sizeof(float)));
+    work.scratch_n = need;
+  }
+}
+bool srce_reserved(const pt::SrceLayout& L, const SrcePlan& plan, const SrceWork& work) {
+  return work.counter != nullptr && static_cast<size_t>(plan.grid) * plan.ns *
+                                            static_cast<size_t>(L.total_g) <= work.scratch_n;
 }
 
 }  // namespace
 
 int srce_max_ctas_per_sm(const pt::SrceLayout& L) {
-  const size_t smem = srce_smem_bytes(L);
-  if (smem == 0) throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
+  if (srce_smem_bytes(L) == 0)
+    throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
   const int keep = g_srce_ctas_per_sm;
   g_srce_ctas_per_sm = 0;
   WWB_CHECK(cudaFuncSetAttribute(srce_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutDefault));
-  const int all = resident_grid(srce_kernel, smem, 1 << 30, kSrceBlock, true) / runtime().sm_count;
+  const int all = srce_per_sm(L, srce_max_slots(L));
   srce_set_ctas_per_sm(L, keep);  // the carveout of the current choice again
   return all;
 }
 
 void srce_set_ctas_per_sm(const pt::SrceLayout& L, int ctas) {
-  const size_t smem = srce_smem_bytes(L);
-  if (smem == 0) throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
+  if (srce_smem_bytes(L) == 0)
+    throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
   g_srce_ctas_per_sm = ctas > 0 ? ctas : 0;
   // The shared-memory carveout just large enough for that many CTAs (their dynamic and static
   // shared memory and the 1 KiB the system keeps per CTA): the rest of the SM's 256 KiB is L1.
   int pct = cudaSharedmemCarveoutDefault;
   if (ctas > 0) {
-    const size_t per_cta = smem + sizeof(pt::SrceSh) + 16 + 1024;
+    const size_t per_cta = srce_smem(L, srce_max_slots(L)) + kSrceStatic + 1024;
     pct = static_cast<int>((100 * ctas * per_cta + 228 * 1024 - 1) / (228 * 1024));
     if (pct > 100) pct = 100;
   }
   WWB_CHECK(cudaFuncSetAttribute(srce_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
-  WWB_CHECK(
-      cudaFuncSetAttribute(srce_multi_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
 }
 
 size_t srce_smem_bytes(const pt::SrceLayout& L) {
-  const size_t b = static_cast<size_t>(L.total_s) * sizeof(float) + 16;
-  return b + sizeof(pt::SrceSh) <= 227 * 1024 ? b : 0;
+  const size_t b = srce_smem(L, 1);
+  return b + kSrceStatic <= 227 * 1024 ? b : 0;
 }
 
 void launch_sds4(const St4Dev* d, const st4::Params& hp, int npts, const float* a, const float* k,
@@ -260,54 +376,25 @@ void launch_spr4(const St4Dev* d, const st4::Params& hp, int npts, const float* 
 
 void srce_reserve(const pt::SrceLayout& L, int npts, SrceWork& work, cudaStream_t st) {
   if (npts <= 0) return;
-  const size_t smem = srce_smem_bytes(L);
-  if (smem == 0) throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
-  const int grid = resident_grid(srce_kernel, smem, npts, kSrceBlock, true);
-  const size_t need = static_cast<size_t>(grid) * static_cast<size_t>(L.total_g);
-  if (work.counter == nullptr) WWB_CHECK(cudaMalloc(&work.counter, sizeof(int)));
-  if (need > work.scratch_n) {
-    WWB_CHECK(cudaStreamSynchronize(st));
-    if (work.scratch) WWB_CHECK(cudaFree(work.scratch));
-    work.scratch = nullptr;
-    work.scratch_n = 0;
-    WWB_CHECK(cudaMalloc(&work.scratch, need * sizeof(float)));
-    work.scratch_n = need;
-  }
-}
-
-int srce_resident_ctas(const pt::SrceLayout& L, int npts) {
-  const size_t smem = srce_smem_bytes(L);
-  if (smem == 0) throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
-  return resident_grid(srce_kernel, smem, npts, kSrceBlock, true);
+  const SrcePlan plan = srce_plan(L, npts);
+  if (srce_reserved(L, plan, work)) return;
+  WWB_CHECK(cudaStreamSynchronize(st));  // earlier launches may still use the old buffers
+  srce_reserve_plan(L, plan, work);
 }
 
 void srce_multi_reserve(const pt::SrceLayout& L, int total, SrceWork& work) {
-  const size_t smem = srce_smem_bytes(L);
-  if (smem == 0) throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
-  const int grid = resident_grid(srce_multi_kernel, smem, total > 0 ? total : 1, kSrceBlock, true);
-  const size_t need = static_cast<size_t>(grid) * static_cast<size_t>(L.total_g);
-  if (work.counter == nullptr) WWB_CHECK(cudaMalloc(&work.counter, sizeof(int)));
-  if (need > work.scratch_n) {
-    if (work.scratch) WWB_CHECK(cudaFree(work.scratch));
-    work.scratch = nullptr;
-    work.scratch_n = 0;
-    WWB_CHECK(cudaMalloc(&work.scratch, need * sizeof(float)));
-    work.scratch_n = need;
-  }
+  srce_reserve_plan(L, srce_plan(L, total > 0 ? total : 1), work);
 }
 
 void launch_srce_multi(const SrceJob* jobs_dev, int njobs, int total, const pt::SrceLayout& L,
                        SrceWork& work, cudaStream_t st) {
   if (total <= 0) return;
-  const size_t smem = srce_smem_bytes(L);
-  if (smem == 0) throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
-  const int grid = resident_grid(srce_multi_kernel, smem, total, kSrceBlock, true);
-  if (work.counter == nullptr ||
-      static_cast<size_t>(grid) * static_cast<size_t>(L.total_g) > work.scratch_n)
+  const SrcePlan plan = srce_plan(L, total);
+  if (!srce_reserved(L, plan, work))
     throw CudaError(cudaErrorInvalidValue, "launch_srce_multi: work buffers not reserved");
   WWB_CHECK(cudaMemsetAsync(work.counter, 0, sizeof(int), st));
-  srce_multi_kernel<<<grid, kSrceBlock, smem, st>>>(jobs_dev, njobs, total, work.counter,
-                                                    work.scratch);
+  srce_kernel<<<plan.grid, kSrceBlock, plan.smem, st>>>(SrceJob{}, jobs_dev, njobs, total, plan.ns,
+                                                        work.counter, work.scratch);
   WWB_CHECK(cudaGetLastError());
 }
 
@@ -316,16 +403,15 @@ void launch_srce(const SrceDev* d, const pt::SrceLayout& L, SrceStep step, int n
                  const float* pin, float* psc, float* whitecap, float* taubbl, float* tauice,
                  int* shave, SrceWork& work, cudaStream_t st) {
   if (npts <= 0) return;
-  const size_t smem = srce_smem_bytes(L);
-  if (smem == 0) throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
-  const int grid = resident_grid(srce_kernel, smem, npts, kSrceBlock, true);
+  const SrcePlan plan = srce_plan(L, npts);
   // The work buffers fit after srce_reserve; otherwise (re)allocate them first, after the
   // previous launches on this stream that may still read the old ones.
   srce_reserve(L, npts, work, st);
   WWB_CHECK(cudaMemsetAsync(work.counter, 0, sizeof(int), st));
-  srce_kernel<<<grid, kSrceBlock, smem, st>>>(d, step, npts, spec, jsea, wn1, cg1, pin, psc,
-                                              whitecap, taubbl, tauice, shave, work.counter,
-                                              work.scratch);
+  const SrceJob job{d,   step, npts, 0,        spec,   jsea,   wn1,  cg1,
+                    pin, psc,  whitecap, taubbl, tauice, shave};
+  srce_kernel<<<plan.grid, kSrceBlock, plan.smem, st>>>(job, nullptr, 1, npts, plan.ns,
+                                                        work.counter, work.scratch);
   WWB_CHECK(cudaGetLastError());
 }
 
