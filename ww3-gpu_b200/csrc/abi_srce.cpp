@@ -54,12 +54,8 @@ struct GridCtx {
   srce::Params p{};
   DevVec<float> sig, dden, ecos, esin;
   DevVec<int> mapwn;
-  SrceDev* dev = nullptr;   ///< device copy of the launch parameters, rebuilt at every call
   SrceWork work;            ///< the work queue's counter, the working sets' global part
-  ~GridCtx() {
-    if (dev) cudaFree(dev);
-    work.release();
-  }
+  ~GridCtx() { work.release(); }
 };
 
 std::map<int, std::unique_ptr<GridCtx>>& grids() {
@@ -101,8 +97,6 @@ bool prepare(int igrid, GridCtx& g, SrceDev& host, const char* who) {
   host.f = q.f;
   host.n = n;
   host.L = pt::srce_layout(q.p, n);
-  if (g.dev == nullptr) WWB_CHECK(cudaMalloc(&g.dev, sizeof(SrceDev)));
-  WWB_CHECK(cudaMemcpy(g.dev, &host, sizeof(SrceDev), cudaMemcpyHostToDevice));
   return true;
 }
 
@@ -147,7 +141,7 @@ void run_batch(int igrid, GridCtx& g, const SrceStep& step, int npts, float* spe
     step_add(
         rec,
         [=](cudaStream_t ss) {
-          launch_srce(d, L, step, npts, va_dev, djsea, dwn, dcg, dpin, dpsc, dwc, dtb, dti, dsh,
+          launch_srce(host, step, npts, va_dev, djsea, dwn, dcg, dpin, dpsc, dwc, dtb, dti, dsh,
                       *w, ss);
         },
         job);
@@ -165,7 +159,7 @@ void run_batch(int igrid, GridCtx& g, const SrceStep& step, int npts, float* spe
   float *dwc = c.in(whitecap, 4 * n, s), *dtb = c.in(taubbl, 2 * n, s),
         *dti = c.in(tauice, 2 * n, s);
   int* dsh = c.in(shave, n, s);
-  launch_srce(g.dev, host.L, step, npts, dspec, djsea, dwn, dcg, dpin, dpsc, dwc, dtb, dti, dsh,
+  launch_srce(host, step, npts, dspec, djsea, dwn, dcg, dpin, dpsc, dwc, dtb, dti, dsh,
               g.work, s);
   if (!va_dev) out(spec, dspec, ns, s);
   out(psc, dpsc, n * srce::NPSC, s);
@@ -361,7 +355,7 @@ void ww_srce_batch_device(int igrid, int it, int inflags24, int flogrd57, int fl
     }
     SrceDev host{};
     if (!prepare(igrid, *g, host, "ww_srce_batch_device")) return;
-    launch_srce(g->dev, host.L, SrceStep{it, inflags24, flogrd57, flogrd58, dtg}, npts, spec,
+    launch_srce(host, SrceStep{it, inflags24, flogrd57, flogrd58, dtg}, npts, spec,
                 nullptr, wn1, cg1, pin, psc, whitecap, taubbl, tauice, shave, g->work,
                 static_cast<cudaStream_t>(stream));
     g_status.ok();
@@ -420,7 +414,7 @@ int ww_srce_autotune(int igrid, int it, int inflags24, int flogrd57, int flogrd5
     const int best = tune::pick(
         key, cands,
         [&](int ctas, cudaStream_t ss) {
-          launch_srce(g->dev, L, step, n, s1.p, nullptr, w.p, c.p, pn.p, q1.p, wc1.p, tb1.p, ti1.p,
+          launch_srce(host, step, n, s1.p, nullptr, w.p, c.p, pn.p, q1.p, wc1.p, tb1.p, ti1.p,
                       reinterpret_cast<int*>(sh.p), g->work, ss);
           (void)ctas;
         },

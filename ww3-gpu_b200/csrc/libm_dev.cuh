@@ -177,6 +177,32 @@ WWB_HD float fma_f(float a, float b, float c) {
 #endif
 }
 
+/// The operations of expf for an argument that is none of its special cases (|x| < 88, and down to
+/// the smallest subnormal result), without their branches.
+WWB_HD float expf_core(float x) {
+  const double xd = (double)x;
+  double kd = fma_d(kInvLn2N, xd, kShift);
+  const uint64_t ki = asuint64(kd);
+  kd -= kShift;
+  const double r = fma_d(kInvLn2N, xd, -kd);
+  uint64_t t = exp2f_tab((unsigned)(ki % 32));
+  t += ki << (52 - 5);
+  const double p = fma_d(kC0, r, kC1);
+  const double r2 = r * r;
+  double y = fma_d(kC2, r, 1.0);
+  y = fma_d(p, r2, y);
+  y = y * asdouble(t);
+  return (float)y;
+}
+/// expf for x < 0.
+WWB_HD float expf_neg(float x) {
+  const float y = expf_core(x);
+  return x < -0x1.9fe368p6f ? 0.0f : y;
+}
+/// expf with the special cases out of line.
+WWB_HD float expf_q(float x) { return x > -80.0f && x < 80.0f ? expf_core(x) : expf(x); }
+static_assert(WWB_EXPF_FUSE == 7, "expf_neg fuses every step");
+
 // ------------------------------------------------------------------------------------ logf
 // 1/c of the 16 subintervals (published table of the method).
 #define WWB_LOG_INVC                                                                          \
@@ -271,6 +297,25 @@ WWB_HD float logf_t(float x) {
 #define WWB_LOGF_FUSE 7
 #endif
 WWB_HC float logf(float x) { return logf_t<WWB_LOGF_FUSE>(x); }
+
+/// logf with the special cases out of line.
+WWB_HD float logf_q(float x) {
+  const uint32_t ix = asuint(x);
+  if (ix - 0x00800000u >= 0x7f800000u - 0x00800000u) return logf(x);
+  const uint32_t tmp = ix - kLogOff;
+  const unsigned i = (tmp >> (23 - 4)) % 16;
+  const int k = (int32_t)tmp >> 23;
+  const double invc = log_invc(i), logc = log_logc(i);
+  const double z = (double)asfloat(ix - (tmp & 0xff800000u));
+  const double r = fma_d(z, invc, -1.0);
+  const double y0 = fma_d((double)k, kLn2, logc);
+  const double r2 = r * r;
+  double y = fma_d(kLogA1, r, kLogA2);
+  y = fma_d(kLogA0, r2, y);
+  y = fma_d(y, r2, y0 + r);
+  return (float)y;
+}
+static_assert(WWB_LOGF_FUSE == 7, "logf_q fuses every step");
 
 // ------------------------------------------------------------------------------------ powf
 // log1p(r)/ln2 ~ A0 r^5 + A1 r^4 + A2 r^3 + A3 r^2 + A4 r (published coefficients).
@@ -380,6 +425,12 @@ WWB_HD float powf_t(float x, float y) {
 #endif
 WWB_HC float powf(float x, float y) { return powf_t<WWB_POWF_FUSE>(x, y); }
 
+/// powf for x in [2^-7, 2) and 0 < y < 16: x is normal and |y log2 x| < 126, so none of the special
+/// cases arises; the same operations without their branches.
+WWB_HD float powf_mid(float x, float y) {
+  return pow_exp2<WWB_POWF_FUSE>((double)y * pow_log2<WWB_POWF_FUSE>(asuint(x)), 0);
+}
+
 // --------------------------------------------------------------------------------- sincosf
 // Cosine 1 + c1 x^2 + ... (c0 = 1) and sine x + s1 x^3 + s2 x^5 + s3 x^7 coefficients of the
 // published method; the second set (quadrants 2, 3) negates the cosine.
@@ -423,15 +474,15 @@ WWB_HD void sincosf_poly(double x, double x2, bool neg, int n, float* sinp, floa
   const double x3 = x2 * x;
   const double cc2 = madd<F>(x2, c4, c3);
   const double ss1 = madd<F>(x2, kScS3, kScS2);
-  float* const sp = (n & 1) ? cosp : sinp;
-  float* const cp = (n & 1) ? sinp : cosp;
   const double cc1 = madd<F>(x2, c1, c0);
   const double x5 = x3 * x2;
   const double x6 = x4 * x2;
   const double s = madd<F>(x3, kScS1, x);
   const double c = madd<F>(x4, c2, cc1);
-  *sp = (float)madd<F>(x5, ss1, s);
-  *cp = (float)madd<F>(x6, cc2, c);
+  // Selected, not stored through exchanged pointers, so the results can stay in registers.
+  const float fs = (float)madd<F>(x5, ss1, s), fc = (float)madd<F>(x6, cc2, c);
+  *sinp = (n & 1) ? fc : fs;
+  *cosp = (n & 1) ? fs : fc;
 }
 
 /// sincosf. FUSE bit 0: the polynomial steps fused; bit 1: x - n*pi/2 fused.
@@ -643,7 +694,7 @@ WWB_HC float coshf(float x) {
 
 // ----------------------------------------------------------------------------- atanf, atan2f
 /// fdlibm atanf.
-WWB_HC float atanf(float x) {
+WWB_HD float atanf_b(float x) {
   const float one = 1.0f, huge = 1.0e30f;
   const float hi0 = asfloat(0x3eed6338u), hi1 = asfloat(0x3f490fdau), hi2 = asfloat(0x3f7b985eu),
               hi3 = asfloat(0x3fc90fdau);
@@ -697,6 +748,8 @@ WWB_HC float atanf(float x) {
   return (hx & 0x80000000u) ? -z : z;
 }
 
+WWB_HC float atanf(float x) { return atanf_b(x); }
+
 /// fdlibm atan2f. KLIM: the |y/x| exponent gap above which the quotient is not formed.
 template <int KLIM>
 WWB_HD float atan2f_t(float y, float x) {
@@ -706,7 +759,7 @@ WWB_HD float atan2f_t(float y, float x) {
   const int32_t ix = hx & 0x7fffffff, iy = hy & 0x7fffffff;
   float z;
   if (ix > 0x7f800000 || iy > 0x7f800000) return x + y;
-  if (hx == 0x3f800000) return atanf(y);
+  if (hx == 0x3f800000) return atanf_b(y);
   const int m = ((hy >> 31) & 1) | ((hx >> 30) & 2);
   if (iy == 0) {
     switch (m) {
@@ -751,7 +804,7 @@ WWB_HD float atan2f_t(float y, float x) {
   } else if (hx < 0 && k < -KLIM) {
     z = 0.0f;
   } else {
-    z = atanf(fabsf(y / x));
+    z = atanf_b(fabsf(y / x));
   }
   switch (m) {
     case 0:

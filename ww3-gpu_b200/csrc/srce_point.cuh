@@ -72,8 +72,10 @@ struct SrceSh {
   int nsteps, nkh, nkh1, nspech, nscut, state, early, done;
   unsigned vmin;      ///< bits of the running MIN of the time-step limits (values >= 0)
   float chains[3];    ///< W3SPR4's ELCS, ELSN, AMAX
+  float c0;           ///< the tail level's factor (:880), a function of the point's CG
+  float stress[2], usdirpl, levtail0, tauhf;  ///< W3SIN4's closing part
   // W3SIN4
-  float uorb, pturb, pvisc, fw, fu, fud, ustarsigma, const1;
+  float fwuorb, pturb, pvisc, fu, fud, ustarsigma, const1;  ///< fwuorb = FW * UORB
   float ust, taux, tauy, cosu, sinu, ustp, cosw, sinw;  ///< cosw, sinw: of the wind direction
   float sums[4];      ///< running STRESS (x, y) and STRESSN (x, y) of one pass
   float ss[3][2], sn[3][2];
@@ -97,6 +99,8 @@ struct SrceLayout {
   int total_g;         ///< floats of global scratch per slot
 };
 
+/// Floats of an array over the tail's steps.
+constexpr int kJtot4 = (kJtot + 3) & ~3;
 /// NK arrays a phase of W3SDS4 / W3SPR4 / W3SIN4 keeps in the transient region.
 constexpr int kNkWork = 20;
 
@@ -120,7 +124,7 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
   int o = 0;
   L.pwsig = o; o += K;
   L.pwdir = o; o += K;
-  L.tail = o; o += r4(6 * kJtot);
+  L.tail = o; o += r4(7 * kJtot + 1);
   L.common = o;
   // Per slot; offsets of slot 0, the others ws further on. SPEC rows start on 16 bytes, and ws is
   // 4 floats more than a multiple of 32, so four lanes reading float4s of four slots meet
@@ -139,7 +143,7 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
   while (L.ws % 32 != 4) L.ws += 4;
   L.tslot = 2 * R + r4((R + 3) / 4) + 8 * K;                  // closing sums + W3SPR4
   if (R + kNkWork * K > L.tslot) L.tslot = R + kNkWork * K;     // W3SDS4
-  const int sin4 = R + r4((R + 3) / 4) + 9 * K;
+  const int sin4 = 2 * R + r4((R + 3) / 4) + 8 * K + 4 * kJtot4;
   if (sin4 > L.tslot) L.tslot = sin4;
   const int seq = 3 * r4(nth) + 9 * K;
   if (seq > L.tslot) L.tslot = seq;
@@ -192,6 +196,15 @@ struct Grp {
   WWB_PD bool role(int r) const { return warp() == r % nwarp(); }
 };
 
+/// In a loop's body: keeps the compiler from making a copy of the loop for each value of the flags that
+/// do not change in it (it does not duplicate what the lanes of a warp agree on). The copies made the
+/// kernel several times larger than the instruction cache.
+WWB_PD void one_copy() {
+#if defined(__CUDA_ARCH__)
+  (void)__activemask();
+#endif
+}
+
 /// Up to kSlots slot numbers, in registers.
 struct SlotList {
   int n = 0;
@@ -203,7 +216,10 @@ struct SlotList {
   WWB_PD int at(int j) const { return (ids >> (4 * j)) & 15; }
 };
 
-/// What the CTA's phases read: the tables of one grid and the slots' memory.
+/// What the CTA's phases read: the tables of one grid and the slots' memory. NTH: the number of
+/// directions where the kernel is built for it (bin addresses and the loops over directions are then
+/// compile-time arithmetic), 0 for any.
+template <int NTH>
 struct SrceGroup {
   const srce::Params* p;
   const SrceGrid* g;
@@ -216,13 +232,16 @@ struct SrceGroup {
   float* t;    ///< the transient region
   SrceSh* sh;  ///< kSlots of them
   int ns;
+  static constexpr int kNth = NTH;
+  WWB_PD int nth() const { return NTH ? NTH : L->nth; }
   WWB_PD float* s(int k, int off) const { return w + off + k * L->ws; }
-  WWB_PD float* gs(int k, int off) const { return gw + off + static_cast<size_t>(k) * L->total_g; }
+  WWB_PD float* gs(int k, int off) const { return gw + (off + k * L->total_g); }
   WWB_PD float* tr(int k) const { return t + k * L->tslot; }
   WWB_PD unsigned char* llws(int k) const {
     return reinterpret_cast<unsigned char*>(w + L->llws + k * L->ws);
   }
   WWB_PD int row(int i) const {
+    if (NTH) return static_cast<int>(static_cast<unsigned>(i) / (NTH ? NTH : 1));
 #if defined(__CUDA_ARCH__)
     return static_cast<int>(__umulhi(static_cast<unsigned>(i), L->nth_magic));
 #else
@@ -231,22 +250,97 @@ struct SrceGroup {
   }
 };
 
+/// f(setup(slot), i) for every bin i < n of the listed slots: a warp takes kLanes consecutive bins
+/// of one slot at a time, slot after slot, so what setup returns (pointers, the point's scalars)
+/// stays in registers. The chunks of all slots are dealt to the warps in one sequence.
+template <class S, class F>
+WWB_PD void bins(const Grp& c, const SlotList& l, int n, S setup, F f) {
+  const int nw = c.nwarp(), nch = (n + Grp::kLanes - 1) / Grp::kLanes, turn = nch % nw;
+  int first = c.warp();
+WWB_UNROLL(1)
+  for (int j = 0; j < l.n; ++j) {
+    const auto s = setup(l.at(j));
+WWB_UNROLL(1)
+    for (int i = first * Grp::kLanes + c.lane(); i < n; i += nw * Grp::kLanes) {
+      one_copy();
+      f(s, i);
+    }
+    first -= turn;
+    if (first < 0) first += nw;
+  }
+}
+/// bins in two stages, U bins of a thread at a time: `ld` reads what a bin needs from global scratch,
+/// `f` does the rest, so U bins' loads are in flight together. `end(s)` follows each slot.
+template <int U, class S, class Ld, class F, class E>
+WWB_PD void bins_ld(const Grp& c, const SlotList& l, int n, S setup, Ld ld, F f, E end) {
+  const int nw = c.nwarp(), nch = (n + Grp::kLanes - 1) / Grp::kLanes, turn = nch % nw;
+  const int step = nw * Grp::kLanes;
+  int first = c.warp();
+WWB_UNROLL(1)
+  for (int j = 0; j < l.n; ++j) {
+    auto s = setup(l.at(j));
+WWB_UNROLL(1)
+    for (int i = first * Grp::kLanes + c.lane(); i < n; i += U * step) {
+      one_copy();
+      decltype(ld(s, i)) in[U];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+      for (int u = 0; u < U; ++u) in[u] = ld(s, i + u * step < n ? i + u * step : i);
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+      for (int u = 0; u < U; ++u)
+        if (i + u * step < n) f(s, i + u * step, in[u]);
+    }
+    end(s);
+    first -= turn;
+    if (first < 0) first += nw;
+  }
+}
+/// f(ith-setup, slot, row) for the nrow rows of every listed slot: a thread keeps its direction, so
+/// what depends on the direction only is formed once.
+template <class S, class F>
+WWB_PD void dirs(const Grp& c, const SlotList& l, int nth, int nrow, S setup, F f) {
+  const bool wide = c.nthr >= nth;
+  const int g = wide ? c.nthr / nth : 1, r0 = wide ? c.tid / nth : 0;
+  if (r0 >= g) return;
+WWB_UNROLL(1)
+  for (int ith = wide ? c.tid - r0 * nth : c.tid; ith < nth; ith += wide ? nth : c.nthr) {
+    const auto s = setup(ith);
+    int j = 0, r = r0;
+    for (;;) {
+      while (r >= nrow && j < l.n) {
+        r -= nrow;
+        ++j;
+      }
+      if (j >= l.n) break;
+      one_copy();
+      f(s, l.at(j), r);
+      r += g;
+    }
+  }
+}
 /// f(slot, i) for every bin i < n of the listed slots: a warp takes kLanes consecutive bins of
 /// one slot, so what depends on the slot only is uniform in the warp.
 template <class F>
 WWB_PD void each_bin(const Grp& c, const SlotList& l, int n, F f) {
   const int nch = (n + Grp::kLanes - 1) / Grp::kLanes, all = l.n * nch;
+WWB_UNROLL(1)
   for (int e = c.warp(); e < all; e += c.nwarp()) {
     const int j = (e >= nch) + (e >= 2 * nch) + (e >= 3 * nch);
     const int i = (e - j * nch) * Grp::kLanes + c.lane();
+    one_copy();
     if (i < n) f(l.at(j), i);
   }
 }
 /// f(slot, r) for r < n of the listed slots, one pair per thread.
 template <class F>
 WWB_PD void each_row(const Grp& c, const SlotList& l, int n, F f) {
+WWB_UNROLL(1)
   for (int e = c.tid; e < l.n * n; e += c.nthr) {
     const int j = (e >= n) + (e >= 2 * n) + (e >= 3 * n);
+    one_copy();
     f(l.at(j), e - j * n);
   }
 }
@@ -254,8 +348,25 @@ static_assert(kSlots <= 4, "each_bin and each_row count three slot boundaries");
 /// f(slot) on warp r: lane k runs the k-th listed slot's chain.
 template <class F>
 WWB_PD void each_chain(const Grp& c, int r, const SlotList& l, F f) {
-  if (c.role(r))
-    for (int j = c.lane(); j < l.n; j += Grp::kLanes) f(l.at(j));
+  if (!c.role(r)) return;
+#if defined(__CUDA_ARCH__)
+  if (c.lane() < l.n) f(l.at(c.lane()));
+#else
+  for (int j = 0; j < l.n; ++j) f(l.at(j));
+#endif
+}
+/// f(r, slot) for nr chains of a kind on warp w, lane r * kSlots + j running chain r of the j-th listed
+/// slot: one instruction serves all of them.
+template <class F>
+WWB_PD void each_chain_of(const Grp& c, int w, int nr, const SlotList& l, F f) {
+  if (!c.role(w)) return;
+#if defined(__CUDA_ARCH__)
+  const int r = c.lane() / kSlots, j = c.lane() % kSlots;
+  if (r < nr && j < l.n) f(r, l.at(j));
+#else
+  for (int r = 0; r < nr; ++r)
+    for (int j = 0; j < l.n; ++j) f(r, l.at(j));
+#endif
 }
 
 struct F4 {
@@ -282,6 +393,7 @@ WWB_UNROLL(4)
     f(v.c, i + 2);
     f(v.d, i + 3);
   }
+WWB_UNROLL(1)
   for (; i < n; ++i) f(x[i], i);
 }
 /// The sum of x[0 .. n) in order from v.
@@ -294,23 +406,42 @@ WWB_PD float row_sum(const float* x, int ik, int nth) {
   const float* const r = x + ik * nth;
   float v = 0.0f;
   if ((nth & 3) == 0) return sum4(r, nth, v);
+WWB_UNROLL(1)
   for (int j = 0; j < nth; ++j) v = v + r[j];
   return v;
 }
 
-WWB_PD float expf_i(float x) { return dm::expf_t<WWB_EXPF_FUSE>(x); }
+/// The sum of the terms whose flag is `want`, in order from v, terms and flags 16- and 4-byte aligned.
+/// The others add -0, which changes no sum: a branch per term would diverge between the slots.
+WWB_PD float sum_flagged(const float* x, const unsigned char* flag, int n, unsigned want, float v) {
+  int i = 0;
+WWB_UNROLL(4)
+  for (; i + 4 <= n; i += 4) {
+    const F4 q = ld4(x + i);
+    const uint32_t b = *reinterpret_cast<const uint32_t*>(flag + i);
+    v = v + ((b & 0xffu) == want ? q.a : -0.0f);
+    v = v + ((b >> 8 & 0xffu) == want ? q.b : -0.0f);
+    v = v + ((b >> 16 & 0xffu) == want ? q.c : -0.0f);
+    v = v + ((b >> 24) == want ? q.d : -0.0f);
+  }
+WWB_UNROLL(1)
+  for (; i < n; ++i) v = v + (flag[i] == want ? x[i] : -0.0f);
+  return v;
+}
+
 WWB_PD float powf_i(float x, float y) { return dm::powf_t<WWB_POWF_FUSE>(x, y); }
-WWB_PD float logf_i(float x) { return dm::logf_t<WWB_LOGF_FUSE>(x); }
 /// Sine and cosine without a call: its results would pass through memory.
 WWB_PD void sincosf_i(float x, float* s, float* c) { dm::sincosf_t<WWB_SINCOSF_FUSE>(x, s, c); }
 
 // ------------------------------------------------------------------ what the slots share
 /// The powers of SIG that W3SPR4 takes and the analytic tail's terms that depend on J only
 /// (:886-917 of W3SIN4): functions of the grid, formed once per CTA.
-WWB_PD void srce_common(const Grp& c, const SrceGroup& x) {
+template <class G>
+WWB_PD void srce_common(const Grp& c, const G& x) {
   const SrceLayout& L = *x.L;
   const st4::Params& q = *x.q;
   const Fields& f = *x.f;
+WWB_UNROLL(1)
   for (int ik = c.tid; ik < L.nk; ik += c.nthr) {
     x.w[L.pwsig + ik] = dm::powf(f.sig[ik + 1], 2.0f * q.wwnmeanptail);
     x.w[L.pwdir + ik] = dm::powf(f.sig[ik + 1], q.ssdsc[11]);
@@ -320,6 +451,7 @@ WWB_PD void srce_common(const Grp& c, const SrceGroup& x) {
     const float signk = f.sig[L.nk];
     const float zinf = dm::logf(signk * signk / kGrav);
     const float dely = (kLogTpiOver005 - zinf) / static_cast<float>(kJtot);
+WWB_UNROLL(1)
     for (int j = c.tid; j < kJtot; j += c.nthr) {
       const float y = dm::expf(zinf + static_cast<float>(j) * dely);
       const float ykm = (y / kKm);
@@ -329,6 +461,9 @@ WWB_PD void srce_common(const Grp& c, const SrceGroup& x) {
       t[j] = cm;
       t[kJtot + j] = 0.5f * (3.0f * ykm2 + 1.0f) * sqrt_f(kGrav / (y * tensk));
       t[4 * kJtot + j] = cm * cm;
+      // 0 where div_by's two steps might not be exact
+      t[6 * kJtot + j] = cm >= 0x1p-20f && cm <= 0x1p20f ? 1.0f / cm : 0.0f;
+      if (j == 0) t[7 * kJtot] = dely;
       t[5 * kJtot + j] = kCmm / cm;
       if (q.sintailpar[2] > 0.0f) {
         const float ykm1 = (ykm - 1.0f);
@@ -343,7 +478,8 @@ WWB_PD void srce_common(const Grp& c, const SrceGroup& x) {
 // ------------------------------------------------------------------ W3SRCE's initialisation
 /// The start of section 1 (:869-1073) for points just loaded: spec, wn1, cg1 and the packets are
 /// in the slots; the slots' state is set.
-WWB_PD void srce_begin(const Grp& c, const SrceGroup& x, const SlotList& l) {
+template <class G>
+WWB_PD void srce_begin(const Grp& c, const G& x, const SlotList& l) {
   const srce::Params& p = *x.p;
   const SrceLayout& L = *x.L;
   each_bin(c, l, L.nspec, [&](int k, int i) {
@@ -369,6 +505,7 @@ WWB_PD void srce_begin(const Grp& c, const SrceGroup& x, const SlotList& l) {
       const float tmax = kTmaxFac / sig;
       const float dt = tmax / 50.0f;
       float mft = 0.0f;
+WWB_UNROLL(1)
       for (int it = 1; it <= 50; ++it) {
         const float t = static_cast<float>(it) * dt;
         if (t < tstr) {
@@ -386,9 +523,10 @@ WWB_PD void srce_begin(const Grp& c, const SrceGroup& x, const SlotList& l) {
     const float depth = mx(x.sh[k].in.d_inp, p.dmin);
     const float* const wn = x.s(k, L.wn1);
     int ik = 0;
+WWB_UNROLL(1)
     for (; ik < L.nk; ++ik)
       if (wn[ik] * depth > 6.0f) break;
-    x.sh[k].nscut = ik == 0 ? -1 : ik * L.nth;
+    x.sh[k].nscut = ik == 0 ? -1 : ik * x.nth();
   });
   each_chain(c, 0, l, [&](int k) {
     SrceSh& s = x.sh[k];
@@ -427,6 +565,12 @@ WWB_PD void srce_begin(const Grp& c, const SrceGroup& x, const SlotList& l) {
     dm::sincosf(in.u10dir, &sn, &cs);
     s.sinw = sn;
     s.cosw = cs;
+    {
+      const float signk = x.f->sig[L.nk];
+      const float s2 = signk * signk;
+      const float s5 = s2 * (s2 * signk);
+      s.c0 = x.q->dth * s5 / kGrav2Tpi * kTpi * signk / x.s(k, L.cg1)[L.nk - 1];
+    }
   });
   c.sync();
 }
@@ -436,15 +580,17 @@ WWB_PD void srce_begin(const Grp& c, const SrceGroup& x, const SlotList& l) {
 /// the terms of the moments (:245-300); the arrays T0 .. T5 and SIGFAC stay in the slot's transient
 /// region from `off` on. The libmvec powers of :316 and :317 use scalar powf in every lane; the
 /// powers are functions of the grid or of the point's WN and are kept (x.w pwsig, pwdir, pwwn).
-WWB_PD void spr4_sums(const Grp& c, const SrceGroup& x, const SlotList& l, int off) {
+template <class G>
+WWB_PD void spr4_sums(const Grp& c, const G& x, const SlotList& l, int off) {
   const SrceLayout& L = *x.L;
   const Fields& f = *x.f;
-  const int nk = L.nk, nth = L.nth;
+  const int nk = L.nk, nth = x.nth();
   each_row(c, l, nk, [&](int k, int ik) {
     const float* const a = x.s(k, L.spec) + ik * nth;
     const unsigned char* const lw = x.llws(k) + ik * nth;
     float ebk = 0.0f, eb2k = 0.0f;
     if ((nth & 3) == 0) {
+WWB_UNROLL(1)
       for (int i = 0; i < nth; i += 4) {
         const F4 v = ld4(a + i);
         const uint32_t b = *reinterpret_cast<const uint32_t*>(lw + i);
@@ -458,6 +604,7 @@ WWB_PD void spr4_sums(const Grp& c, const SrceGroup& x, const SlotList& l, int o
         if (b & 0xff000000u) eb2k = eb2k + v.d;
       }
     } else {
+WWB_UNROLL(1)
       for (int i = 0; i < nth; ++i) {
         ebk = ebk + a[i];
         if (lw[i] != 0) eb2k = eb2k + a[i];
@@ -480,11 +627,12 @@ WWB_PD void spr4_sums(const Grp& c, const SrceGroup& x, const SlotList& l, int o
 /// Second phase, roles 0-3: the moments with CALC_USTAR, and the running sums ELCS, ELSN and the
 /// running MAX over all bins. Each chain is 5 k cycles at 36 x 36 and the moments 15 k (ten Newton
 /// steps of CALC_USTAR); side by side they cost the longest one.
-WWB_PD void spr4_chains(const Grp& c, const SrceGroup& x, const SlotList& l, int off) {
+template <class G>
+WWB_PD void spr4_chains(const Grp& c, const G& x, const SlotList& l, int off) {
   const SrceLayout& L = *x.L;
   const st4::Params& p = *x.q;
   const Fields& f = *x.f;
-  const int nk = L.nk, nth = L.nth;
+  const int nk = L.nk, nth = x.nth();
   each_chain(c, 0, l, [&](int k) {
     SrceSh& s = x.sh[k];
     const float* const t = x.tr(k) + off;
@@ -540,22 +688,33 @@ WWB_UNROLL(4)
     s.r.charn = charn;
     s.r.fmeanws = fmeanws;
   });
-  for (int comp = 0; comp < 2; ++comp) {
-    each_chain(c, 1 + comp, l, [&](int k) {
+WWB_UNROLL(1)
+  each_chain_of(c, 1, 2, l, [&](int comp, int k) {
       const float* const a = x.s(k, L.spec);
       const float* const sf = x.tr(k) + off + 6 * nk;
       const float* const e = comp ? f.esin : f.ecos;
       float v = 0.0f;
+WWB_UNROLL(1)
       for (int ik = 0; ik < nk; ++ik) {
         const float sfk = sf[ik];
         const float* const ar = a + ik * nth;
         const float* const er = e + ik * nth;
-WWB_UNROLL(12)
-        for (int i = 0; i < nth; ++i) v = v + ar[i] * er[i] * sfk;
+        int i = 0;
+        if ((nth & 3) == 0) {
+WWB_UNROLL(3)
+          for (; i < nth; i += 4) {
+            const F4 q = ld4(ar + i), r = ld4(er + i);
+            v = v + q.a * r.a * sfk;
+            v = v + q.b * r.b * sfk;
+            v = v + q.c * r.c * sfk;
+            v = v + q.d * r.d * sfk;
+          }
+        }
+WWB_UNROLL(1)
+        for (; i < nth; ++i) v = v + ar[i] * er[i] * sfk;
       }
       x.sh[k].chains[comp] = v;
     });
-  }
   each_chain(c, 3, l, [&](int k) {
     float v = 0.0f;
     walk4(x.s(k, L.spec), L.nspec, [&](float a, int) { v = max_r(v, a); });
@@ -568,50 +727,52 @@ WWB_UNROLL(12)
 struct ScanK {
   float cm, ucn, const2, cnst, zcn, swv, swt, sig2is;
 };
-/// DSTAB and LLWS of one bin (:739-783).
-WWB_PD float scan_bin(const st4::Params& p, const SrceSh& s, const ScanK& q, float ustar,
+/// DSTAB and LLWS of one bin (:739-783). `plain`: 0 < SSINTHP < 16, so that COS**SSINTHP (a cosine
+/// between 0.01 and 1) and the exponential need no special case and the bins of a thread overlap.
+template <class S>
+WWB_PD float scan_bin(const st4::Params& p, const S& s, const ScanK& q, bool plain, float ustar,
                       float ustp, float coswind, int* lw) {
-  float dst;
-  if (coswind > 0.01f) {
-    const float xx = coswind * q.ucn;
-    const float zarg = kKappa / xx;
-    const float zlog = q.zcn + zarg;
-    int l;
-    if (zlog < 0.0f) {
-      const float zlog2 = zlog * zlog;
-      dst = q.cnst * expf_i(zlog) * (zlog2 * zlog2) * q.ucn * q.ucn * powf_i(coswind, p.ssinthp);
-      l = 1;
-    } else {
-      dst = 0.0f;
-      l = 0;
-    }
-    if (28.0f * q.cm * ustar * coswind >= 1.0f) l = 1;
-    *lw = l;
-  } else {
-    dst = 0.0f;
-    *lw = 0;
+  const bool up = coswind > 0.01f;
+  const float xx = coswind * q.ucn;
+  const float zarg = kKappa / xx;
+  const float zlog = q.zcn + zarg;
+  const bool grow = up && zlog < 0.0f;
+  float dst = 0.0f;
+  if (plain) {
+    const float zl = grow ? zlog : -1.0f, cw = grow ? coswind : 0.5f;
+    const float zlog2 = zl * zl;
+    const float g = q.cnst * dm::expf_neg(zl) * (zlog2 * zlog2) * q.ucn * q.ucn *
+                    dm::powf_mid(cw, p.ssinthp);
+    dst = grow ? g : 0.0f;
+  } else if (grow) {
+    const float zlog2 = zlog * zlog;
+    dst = q.cnst * dm::expf(zlog) * (zlog2 * zlog2) * q.ucn * q.ucn * dm::powf(coswind, p.ssinthp);
   }
+  *lw = grow || (up && 28.0f * q.cm * ustar * coswind >= 1.0f) ? 1 : 0;
   if ((p.sswellf[0] != 0.0f && dst < 1E-7f * q.sig2is) || p.sswellf[2] > 0.0f) {
     const float dvisc = q.swv;
-    const float dturb = q.swt * (s.fw * s.uorb + (s.fu + s.fud * coswind) * ustp);
+    const float dturb = q.swt * (s.fwuorb + (s.fu + s.fud * coswind) * ustp);
     dst = dst + s.pturb * dturb + s.pvisc * dvisc;
   }
   return dst;
 }
+WWB_PD bool scan_plain(const st4::Params& p) { return p.ssinthp > 0.0f && p.ssinthp < 16.0f; }
 
-/// Offsets of W3SIN4's NK arrays in a slot's transient region (after the R + R/4 floats of the
+/// Offsets of W3SIN4's NK arrays in a slot's transient region (after the 2 R + R/4 floats of the
 /// stress terms and their signs).
 struct Sin4At {
-  int zcn, cm, const2, cnst, swv, swt, tu, ta, end;
+  int zcn, cm, const2, cnst, swv, swt, tu, ta, gz, zb, us, lev;
 };
 WWB_PD Sin4At sin4_at(const SrceLayout& L) {
   const int R = (L.nspec + 3) & ~3, K = (L.nk + 3) & ~3;
-  const int o = R + ((((R + 3) / 4) + 3) & ~3);
-  return Sin4At{o, o + K, o + 2 * K, o + 3 * K, o + 4 * K, o + 5 * K, o + 6 * K, o + 7 * K, o + 8 * K};
+  const int o = 2 * R + ((((R + 3) / 4) + 3) & ~3);
+  return Sin4At{o, o + K, o + 2 * K, o + 3 * K, o + 4 * K, o + 5 * K, o + 6 * K, o + 7 * K, o + 8 * K,
+                o + 8 * K + kJtot4, o + 8 * K + 2 * kJtot4, o + 8 * K + 3 * kJtot4};
 }
 
-WWB_PD ScanK scan_k(const SrceGroup& x, const Sin4At& at, int k, int ik, float ustp) {
-  const float* const t = x.tr(k) + ik;
+template <class G>
+WWB_PD ScanK scan_k(const G& x, const Sin4At& at, const float* tr, int ik, float ustp) {
+  const float* const t = tr + ik;
   ScanK q;
   q.cm = t[at.cm];
   q.ucn = ustp * q.cm + x.q->zzalp;
@@ -620,7 +781,7 @@ WWB_PD ScanK scan_k(const SrceGroup& x, const Sin4At& at, int k, int ik, float u
   q.zcn = t[at.zcn];
   q.swv = t[at.swv];
   q.swt = t[at.swt];
-  q.sig2is = x.f->sig2[ik * x.L->nth];
+  q.sig2is = x.f->sig2[ik * x.nth()];
   return q;
 }
 
@@ -636,13 +797,16 @@ constexpr int kScanLanes = 1;
 /// (TTAUWSHELTER /= 0) or that the parallel form leaves to it. A team of kScanLanes lanes takes one
 /// point: every lane forms the frequency's scalars, the directions are split, and the four ordered
 /// sums (x and y, by the sign of DSTAB) are one lane each.
-WWB_PD void scan_serial(const Grp& c, const SrceGroup& x, const SlotList& l, const Sin4At& at) {
+template <class G>
+WWB_PD void scan_serial(const Grp& c, const G& x, const SlotList& l, const Sin4At& at) {
   const SrceLayout& L = *x.L;
   const st4::Params& p = *x.q;
   const Fields& f = *x.f;
-  const int nk = L.nk, nth = L.nth, T4 = (nth + 3) & ~3;
+  const int nk = L.nk, nth = x.nth(), T4 = (nth + 3) & ~3;
+  const bool plain = scan_plain(p);
   constexpr int kPerWarp = Grp::kLanes / kScanLanes;
   const int team = c.lane() / kScanLanes, sub = c.lane() - team * kScanLanes;
+WWB_UNROLL(1)
   for (int j0 = c.warp() * kPerWarp; j0 < l.n; j0 += c.nwarp() * kPerWarp) {
     const int j = j0 + team;
     const bool on = team < kPerWarp && j < l.n;
@@ -655,31 +819,39 @@ WWB_PD void scan_serial(const Grp& c, const SrceGroup& x, const SlotList& l, con
     const float* const a = x.s(k, L.spec);
     unsigned char* const llws = x.llws(k);
     float* const vdin = x.gs(k, L.vdin);
+    struct Swell {
+      float fwuorb, fu, fud, pturb, pvisc;
+    };
+    const Swell sw{s.fwuorb, s.fu, s.fud, s.pturb, s.pvisc};
     const float ustar = s.r.ustar, shelter = fabs_f(p.ttauwshelter);
     float ust = ustar, taux = 0.0f, tauy = 0.0f, cosu = 0.0f, sinu = 0.0f, ustp = 0.0f;
     const int first = p.stab3 ? 1 : 3, last = p.stab3 ? 2 : 3;
+WWB_UNROLL(1)
     for (int istab = first; istab <= last; ++istab) {
       if (istab == 1) ust = ustar * (1.0f - s.ustarsigma);
       if (istab == 2) ust = ustar * (1.0f + s.ustarsigma);
       taux = (ust * ust) * s.cosw;
       tauy = (ust * ust) * s.sinw;
       if (on)
+WWB_UNROLL(1)
         for (int q = sub; q < 4; q += kScanLanes) s.sums[q] = 0.0f;
       c.syncwarp();
+WWB_UNROLL(1)
       for (int ik = 0; ik < nk; ++ik) {
         if (on) {
           const float taupx = taux - shelter * s.sums[0];
           const float taupy = tauy - shelter * s.sums[1];
           ustp = min_r(powf_i((taupx * taupx + taupy * taupy), 0.25f), max_r(ust, 0.3f));
-          const float usdirp = dm::atan2f(taupy, taupx);
+          const float usdirp = dm::atan2f_t<WWB_ATAN2F_KLIM>(taupy, taupx);
           sincosf_i(usdirp, &sinu, &cosu);
-          const ScanK q = scan_k(x, at, k, ik, ustp);
+          const ScanK q = scan_k(x, at, t, ik, ustp);
+WWB_UNROLL(3)
           for (int ith = sub; ith < nth; ith += kScanLanes) {
             const int i = ik * nth + ith;
             const float ecos = f.ecos[i], esin = f.esin[i];
             const float coswind = (ecos * cosu + esin * sinu);
             int lw;
-            const float dst = scan_bin(p, s, q, ustar, ustp, coswind, &lw);
+            const float dst = scan_bin(p, sw, q, plain, ustar, ustp, coswind, &lw);
             if (istab == 2) {
               vdin[i] = 0.5f * (vdin[i] + dst);
             } else {
@@ -694,14 +866,9 @@ WWB_PD void scan_serial(const Grp& c, const SrceGroup& x, const SlotList& l, con
         }
         c.syncwarp();
         if (on)
+WWB_UNROLL(1)
           for (int q = sub; q < 4; q += kScanLanes) {
-            float v = s.sums[q];
-            const float* const b = (q & 1) ? by : bx;
-            const unsigned want = static_cast<unsigned>(q >> 1);
-WWB_UNROLL(12)
-            for (int ith = 0; ith < nth; ++ith)
-              if (neg[ith] == want) v = v + b[ith];
-            s.sums[q] = v;
+            s.sums[q] = sum_flagged((q & 1) ? by : bx, neg, nth, static_cast<unsigned>(q >> 1), s.sums[q]);
           }
         c.syncwarp();
       }
@@ -724,16 +891,149 @@ WWB_UNROLL(12)
   }
 }
 
+/// a / b for b in [2^-20, 2^20], correctly rounded, from y = 1 / b correctly rounded (0: unknown): two steps q + (a - b q) y with fused
+/// multiply-adds (Markstein 1990, IBM J. Res. Dev. 34: one step from a quotient within an ulp is exact,
+/// the first makes it so), where nothing under- or overflows; else the division itself. The tail divides
+/// by the same 50 phase speeds in every substep, and this is a third of a division's latency.
+WWB_PD float div_by(float a, float b, float y) {
+  const float m = fabs_f(a);
+  if (!((m >= 0x1p-80f && m <= 0x1p80f || a == 0.0f) && y != 0.0f)) return a / b;
+  float q = a * y;
+  q = dm::fma_f(dm::fma_f(-b, q, a), y, q);
+  return dm::fma_f(dm::fma_f(-b, q, a), y, q);
+}
+
+/// The serial part of W3SIN4's closing section for one slot (:799-955): the stresses, the tail's level
+/// and the tail's recurrence (per step ZBETA and USTR**2 are kept, TAU1 is summed afterwards), or the
+/// tabulated tail. 50 dependent steps of an exponential, a logarithm, a division and a square root: the
+/// longest chain of a substep, so what does not depend on the step before is taken out of it.
+template <class G>
+WWB_PD void sin4_tail(const G& x, int k, const Sin4At& at) {
+  const SrceLayout& L = *x.L;
+  const st4::Params& p = *x.q;
+  const Fields& f = *x.f;
+  const int nk = L.nk, nth = x.nth();
+  SrceSh& s = x.sh[k];
+  const float* const a = x.s(k, L.spec) + (nk - 1) * nth;
+  float xstress, ystress, twnx, twny;
+  if (!p.stab3) {
+    xstress = s.ss[2][0];
+    ystress = s.ss[2][1];
+    twnx = s.sn[2][0];
+    twny = s.sn[2][1];
+  } else {
+    xstress = 0.5f * (s.ss[0][0] + s.ss[1][0]);
+    ystress = 0.5f * (s.ss[0][1] + s.ss[1][1]);
+    twnx = 0.5f * (s.sn[0][0] + s.sn[1][0]);
+    twny = 0.5f * (s.sn[0][1] + s.sn[1][1]);
+  }
+  s.tauwax = twnx;
+  s.tauway = twny;
+  s.stress[0] = xstress;
+  s.stress[1] = ystress;
+  float ustl;
+  {
+    const float taupx = s.taux - fabs_f(p.ttauwshelter) * xstress;
+    const float taupy = s.tauy - fabs_f(p.ttauwshelter) * ystress;
+    ustl = dm::powf((taupx * taupx + taupy * taupy), 0.25f);
+    s.usdirpl = dm::atan2f(taupy, taupx);
+  }
+  const float ust3 = ustl, z0 = s.r.z0;
+  float temp = 0.0f;
+  {
+    const float cosu = s.cosu, sinu = s.sinu;
+    const float *const ec = f.ecos + (nk - 1) * nth, *const es = f.esin + (nk - 1) * nth;
+WWB_UNROLL(6)
+    for (int i = 0; i < nth; ++i) {
+      const float coswind = (ec[i] * cosu + es[i] * sinu);
+      const float cp = (max_r(coswind, 0.0f));
+      temp = temp + a[i] * (cp * (cp * cp));
+    }
+  }
+  const float levtail0 = s.c0 * temp;
+  s.levtail0 = levtail0;
+  if (p.sintailpar[0] < 0.5f) {
+    const float* const tt = x.w + L.tail;
+    float* const tr = x.tr(k);
+    float ustr = ust3;
+    const float dely = tt[7 * kJtot];
+    float taur = ust3 * ust3;
+    const float const1 = s.const1, zzalp = p.zzalp, sp1 = p.sintailpar[1];
+    const bool lev = p.sintailpar[2] > 0.0f;
+WWB_UNROLL(1)
+    for (int j = 0; j < kJtot; ++j) {
+      one_copy();
+      const float cm = tt[j], cgtail = tt[kJtot + j], rcm = tt[6 * kJtot + j];
+      const float zx = div_by(ustr, cm, rcm) + zzalp;
+      const float zarg = min_r(kKappa / zx, 20.0f);
+      const float zmu = min_r(tr[at.gz + j] * dm::expf_q(zarg), 1.0f);
+      const float zlog = min_r(dm::logf_q(zmu), 0.0f);
+      const float zlog2 = zlog * zlog;
+      const float zbeta = const1 * zmu * (zlog2 * zlog2);
+      float levtail = levtail0;
+      if (lev) {
+        float alpham;
+        if (ustr < cm) {
+          alpham = max_r(0.0f, 0.01f * (1.0f + dm::logf(ustr / cm)));
+        } else {
+          alpham = 0.01f * (1.0f + 3.0f * dm::logf(ustr / cm));
+        }
+        const float fm = tt[2 * kJtot + j];
+        const float alphat = alpham * tt[5 * kJtot + j] * fm;
+        const float th = tt[3 * kJtot + j];
+        levtail = levtail0 * 0.5f * (1.0f - th) + p.sintailpar[2] * 0.5f * (1.0f + th) * alphat;
+        tr[at.lev + j] = levtail;
+      }
+      const float us2 = ustr * ustr, w = (j == 0 || j == kJtot - 1) ? 0.5f : 1.0f;
+      tr[at.zb + j] = zbeta;
+      tr[at.us + j] = us2;
+      taur = taur - div_by(w * sp1 * us2 * zbeta * levtail * dely * cgtail, cm, rcm);
+      ustr = sqrt_f(max_r(taur, 0.0f));
+    }
+  } else {
+    const float xi = ust3 / p.delust;
+    const int ind = max_i(1, min_i(st4::kIustar - 1, fint(xi)));
+    const float deli1 = max_r(min_r(1.0f, xi - static_cast<float>(ind)), 0.0f);
+    const float deli2 = 1.0f - deli1;
+    const float ustm = max_r(ust3, 0.00001f);
+    const float xj = max_r(0.0f, (kGrav * z0 / (ustm * ustm) - p.aalpha) / p.delalp);
+    const int j = max_i(1, min_i(st4::kIalpha - 1, fint(xj)));
+    const float delj1 = max_r(0.0f, min_r(1.0f, xj - static_cast<float>(j)));
+    const float delj2 = 1.0f - delj1;
+    float tau1;
+    if (p.ttauwshelter > 0.0f) {
+      const float xk = levtail0 / p.deltail;
+      const int i = min_i(st4::kIlevTail - 1, fint(xk));
+      const float delk1 = min_r(1.0f, xk - static_cast<float>(i));
+      const float delk2 = 1.0f - delk1;
+      tau1 = ((f.tauhft2_at(ind, j, i) * deli2 + f.tauhft2_at(ind + 1, j, i) * deli1) * delj2 +
+              (f.tauhft2_at(ind, j + 1, i) * deli2 + f.tauhft2_at(ind + 1, j + 1, i) * deli1) *
+                  delj1) * delk2 +
+             ((f.tauhft2_at(ind, j, i + 1) * deli2 + f.tauhft2_at(ind + 1, j, i + 1) * deli1) *
+                  delj2 +
+              (f.tauhft2_at(ind, j + 1, i + 1) * deli2 +
+               f.tauhft2_at(ind + 1, j + 1, i + 1) * deli1) *
+                  delj1) *
+                 delk1;
+    } else {
+      tau1 = (f.tauhft_at(ind, j) * deli2 + f.tauhft_at(ind + 1, j) * deli1) * delj2 +
+             (f.tauhft_at(ind, j + 1) * deli2 + f.tauhft_at(ind + 1, j + 1) * deli1) * delj1;
+    }
+    s.tauhf = levtail0 * (ust3 * ust3) * tau1;
+  }
+}
+
 WWB_PD bool finite_f(float v) { return fabs_f(v) <= 3.402823466e38f; }
 
 /// W3SIN4 (w3src4md.F90:423-1003) of the listed slots with W3SRCE's arguments (:1100, :1239, :2007):
 /// VDIN, LLWS, TAUWX/Y, TAUWAX/Y. VSIN = VDIN * SPEC is formed where it is read (the spectrum does not
 /// change before that).
-WWB_PD void srce_sin4(const Grp& c, const SrceGroup& x, const SlotList& l) {
+template <class G>
+WWB_PD void srce_sin4(const Grp& c, const G& x, const SlotList& l) {
   const SrceLayout& L = *x.L;
   const st4::Params& p = *x.q;
   const Fields& f = *x.f;
-  const int nk = L.nk, nth = L.nth;
+  const int nk = L.nk, nth = x.nth();
   const Sin4At at = sin4_at(L);
   // 1. Preparations (:600-675).
   each_row(c, l, nk, [&](int k, int ik) {
@@ -746,12 +1046,16 @@ WWB_PD void srce_sin4(const Grp& c, const SrceGroup& x, const SlotList& l) {
     t[at.cm] = kis / sig2is;
     t[at.const2] = f.dden2[ik * nth] / cg * kGrav / (sigk / kis * s.drat);
     t[at.cnst] = sig2is * const0;
-    t[at.zcn] = logf_i(kis * s.r.z0);
+    t[at.zcn] = dm::logf_q(kis * s.r.z0);
     t[at.swv] = -(p.sswellf[4] * s.drat * 2.0f * kis * sqrt_f(kTwoNuAir * sig2is));
     t[at.swt] = -(s.drat * p.sswellf[0] * 16.0f * (sig2is * sig2is) / kGrav);
     t[at.tu] = e * (sigk * sigk) * f.dden[ik] / cg;
     t[at.ta] = e * f.dden[ik] / cg;
   });
+  if (p.sintailpar[0] < 0.5f)
+    each_row(c, l, kJtot, [&](int k, int j) {
+      x.tr(k)[at.gz + j] = kGrav * x.sh[k].r.z0 / x.w[L.tail + 4 * kJtot + j];
+    });
   c.sync();
   each_chain(c, 0, l, [&](int k) {
     SrceSh& s = x.sh[k];
@@ -812,10 +1116,9 @@ WWB_UNROLL(4)
       ustarsigma = (1.0f + s.in.u10abs / (10.0f + s.in.u10abs)) * usigma;
     }
     s.const1 = const1;
-    s.uorb = uorb;
+    s.fwuorb = fw * uorb;
     s.pturb = pturb;
     s.pvisc = pvisc;
-    s.fw = fw;
     s.fu = fu;
     s.fud = fud;
     s.ustarsigma = ustarsigma;
@@ -845,41 +1148,50 @@ WWB_UNROLL(4)
   c.sync();
   // 2. The stress scan over IK (:696-797).
   SlotList par, ser;
+WWB_UNROLL(1)
   for (int j = 0; j < l.n; ++j) {
     if (x.sh[l.at(j)].scan_par) par.add(l.at(j));
     else ser.add(l.at(j));
   }
   if (par.n) {
     const int R = (L.nspec + 3) & ~3;
-    each_bin(c, par, L.nspec, [&](int k, int i) {
+    const bool plain = scan_plain(p);
+    struct Slot {
+      const float* spec;
+      float *vdin, *t;
+      const float* tk;
+      unsigned char *llws, *neg;
+      float ustar, ustp, cosu, sinu, fwuorb, fu, fud, pturb, pvisc;
+    };
+    bins(c, par, L.nspec, [&](int k) {
       const SrceSh& s = x.sh[k];
+      return Slot{x.s(k, L.spec), x.gs(k, L.vdin), x.tr(k), x.tr(k), x.llws(k),
+                  reinterpret_cast<unsigned char*>(x.tr(k) + 2 * R), s.r.ustar, s.ustp, s.cosu, s.sinu,
+                  s.fwuorb, s.fu, s.fud, s.pturb, s.pvisc};
+    }, [&](const Slot& s, int i) {
       const int ik = x.row(i);
-      const float ustp = s.ustp;
-      const ScanK q = scan_k(x, at, k, ik, ustp);
-      const float coswind = (f.ecos[i] * s.cosu + f.esin[i] * s.sinu);
+      const ScanK q = scan_k(x, at, s.tk, ik, s.ustp);
+      const float ecos = f.ecos[i], esin = f.esin[i];
+      const float coswind = (ecos * s.cosu + esin * s.sinu);
       int lw;
-      const float dst = scan_bin(p, s, q, s.r.ustar, ustp, coswind, &lw);
-      x.gs(k, L.vdin)[i] = dst;
-      x.llws(k)[i] = static_cast<unsigned char>(lw);
-      x.tr(k)[i] = q.const2 * dst * x.s(k, L.spec)[i];
-      reinterpret_cast<unsigned char*>(x.tr(k) + R)[i] = dst < 0.0f ? 1 : 0;
+      const float dst = scan_bin(p, s, q, plain, s.ustar, s.ustp, coswind, &lw);
+      s.vdin[i] = dst;
+      s.llws[i] = static_cast<unsigned char>(lw);
+      const float temp2 = q.const2 * dst * s.spec[i];
+      s.t[i] = temp2 * ecos;
+      s.t[R + i] = temp2 * esin;
+      s.neg[i] = dst < 0.0f ? 1 : 0;
     });
     c.sync();
-    for (int r = 0; r < 4; ++r) {
-      each_chain(c, r, par, [&](int k) {
-        const float* const e = (r & 1) ? f.esin : f.ecos;
-        const float* const t2 = x.tr(k);
-        const unsigned char* const neg = reinterpret_cast<const unsigned char*>(t2 + R);
-        const unsigned want = static_cast<unsigned>(r >> 1);
-        float v = 0.0f;
-        walk4(t2, L.nspec, [&](float tv, int i) {
-          if (neg[i] == want) v = v + tv * e[i];
-        });
+    each_chain_of(c, 0, 4, par, [&](int r, int k) {
+        const float* const t = x.tr(k);
+        const float v = sum_flagged(t + (r & 1) * R, reinterpret_cast<const unsigned char*>(t + 2 * R),
+                                    L.nspec, static_cast<unsigned>(r >> 1), 0.0f);
         x.sh[k].sums[r] = v;
         (r < 2 ? x.sh[k].ss : x.sh[k].sn)[2][r & 1] = v;
-      });
-    }
+    });
     c.sync();
+WWB_UNROLL(1)
     for (int j = 0; j < par.n; ++j) {
       const SrceSh& s = x.sh[par.at(j)];
       if (!finite_f(s.sums[0]) || !finite_f(s.sums[1])) ser.add(par.at(j));
@@ -890,134 +1202,51 @@ WWB_UNROLL(4)
     scan_serial(c, x, ser, at);
     c.sync();
   }
-  // 3. The tail stress and the stress limit (:799-976).
-  each_chain(c, 0, l, [&](int k) {
-    SrceSh& s = x.sh[k];
-    const float* const a = x.s(k, L.spec);
-    float xstress, ystress, twnx, twny;
-    if (!p.stab3) {
-      xstress = s.ss[2][0];
-      ystress = s.ss[2][1];
-      twnx = s.sn[2][0];
-      twny = s.sn[2][1];
-    } else {
-      xstress = 0.5f * (s.ss[0][0] + s.ss[1][0]);
-      ystress = 0.5f * (s.ss[0][1] + s.ss[1][1]);
-      twnx = 0.5f * (s.sn[0][0] + s.sn[1][0]);
-      twny = 0.5f * (s.sn[0][1] + s.sn[1][1]);
+  // 3. The tail stress and the stress limit (:799-976), one warp.
+  if (c.role(0)) {
+WWB_UNROLL(1)
+    for (int j = c.lane(); j < l.n; j += Grp::kLanes) {
+      one_copy();
+      sin4_tail(x, l.at(j), at);
     }
-    s.tauwax = twnx;
-    s.tauway = twny;
-    float ustl, usdirpl;
-    {
-      const float taupx = s.taux - fabs_f(p.ttauwshelter) * xstress;
-      const float taupy = s.tauy - fabs_f(p.ttauwshelter) * ystress;
-      ustl = dm::powf((taupx * taupx + taupy * taupy), 0.25f);
-      usdirpl = dm::atan2f(taupy, taupx);
-    }
-    const float ust3 = ustl, z0 = s.r.z0, ustar = s.r.ustar;
-    float c0;
-    {
-      const float signk = f.sig[nk];
-      const float s2 = signk * signk;
-      const float s5 = s2 * (s2 * signk);
-      c0 = p.dth * s5 / kGrav2Tpi * kTpi * signk / x.s(k, L.cg1)[nk - 1];
-    }
-    float temp = 0.0f;
-    for (int ith = 0; ith < nth; ++ith) {
-      const int i = ith + (nk - 1) * nth;
-      const float coswind = (f.ecos[i] * s.cosu + f.esin[i] * s.sinu);
-      const float cp = (max_r(coswind, 0.0f));
-      temp = temp + a[i] * (cp * (cp * cp));
-    }
-    const float levtail0 = c0 * temp;
-    float tauhf;
+    c.syncwarp();
     if (p.sintailpar[0] < 0.5f) {
-      const float* const tt = x.w + L.tail;
-      float ustr = ust3;
-      const float signk = f.sig[nk];
-      const float zinf = dm::logf(signk * signk / kGrav);
-      const float dely = (kLogTpiOver005 - zinf) / static_cast<float>(kJtot);
-      float taur = ust3 * ust3;
-      float tau1 = 0.0f;
-      const float const1 = s.const1, gz0 = kGrav * z0;
-      for (int j = 1; j <= kJtot; ++j) {
-        const float w = (j == 1 || j == kJtot) ? 0.5f : 1.0f;
-        const float cm = tt[j - 1];
-        const float cgtail = tt[kJtot + j - 1];
-        const float gz = gz0 / tt[4 * kJtot + j - 1];
-        const float zx = ustr / cm + p.zzalp;
-        const float zarg = min_r(kKappa / zx, 20.0f);
-        const float zmu = min_r(gz * expf_i(zarg), 1.0f);
-        const float zlog = min_r(logf_i(zmu), 0.0f);
-        const float zlog2 = zlog * zlog;
-        const float zbeta = const1 * zmu * (zlog2 * zlog2);
-        float levtail;
-        if (p.sintailpar[2] > 0.0f) {
-          float alpham;
-          if (ustr < cm) {
-            alpham = max_r(0.0f, 0.01f * (1.0f + dm::logf(ustr / cm)));
-          } else {
-            alpham = 0.01f * (1.0f + 3.0f * dm::logf(ustr / cm));
-          }
-          const float fm = tt[2 * kJtot + j - 1];
-          const float alphat = alpham * tt[5 * kJtot + j - 1] * fm;
-          const float th = tt[3 * kJtot + j - 1];
-          levtail = levtail0 * 0.5f * (1.0f - th) + p.sintailpar[2] * 0.5f * (1.0f + th) * alphat;
-        } else {
-          levtail = levtail0;
-        }
-        tau1 = tau1 + w * zbeta * (ustr * ustr) * levtail * dely * cgtail / cm;
-        taur = taur - w * p.sintailpar[1] * (ustr * ustr) * zbeta * levtail * dely * cgtail / cm;
-        ustr = sqrt_f(max_r(taur, 0.0f));
+      // TAU1's terms: they do not feed the next step of the tail, so they are formed side by side.
+      const float dely = x.w[L.tail + 7 * kJtot];
+WWB_UNROLL(1)
+      for (int e = c.lane(); e < l.n * kJtot; e += Grp::kLanes) {
+        const int n = (e >= kJtot) + (e >= 2 * kJtot) + (e >= 3 * kJtot), k = l.at(n), j = e - n * kJtot;
+        float* const t = x.tr(k);
+        const float w = (j == 0 || j == kJtot - 1) ? 0.5f : 1.0f;
+        const float lev = p.sintailpar[2] > 0.0f ? t[at.lev + j] : x.sh[k].levtail0;
+        t[at.zb + j] = w * t[at.zb + j] * t[at.us + j] * lev * dely * x.w[L.tail + kJtot + j] /
+                       x.w[L.tail + j];
       }
-      tauhf = tau1;
-    } else {
-      const float xi = ust3 / p.delust;
-      const int ind = max_i(1, min_i(st4::kIustar - 1, fint(xi)));
-      const float deli1 = max_r(min_r(1.0f, xi - static_cast<float>(ind)), 0.0f);
-      const float deli2 = 1.0f - deli1;
-      const float ustm = max_r(ust3, 0.00001f);
-      const float xj = max_r(0.0f, (kGrav * z0 / (ustm * ustm) - p.aalpha) / p.delalp);
-      const int j = max_i(1, min_i(st4::kIalpha - 1, fint(xj)));
-      const float delj1 = max_r(0.0f, min_r(1.0f, xj - static_cast<float>(j)));
-      const float delj2 = 1.0f - delj1;
-      float tau1;
-      if (p.ttauwshelter > 0.0f) {
-        const float xk = levtail0 / p.deltail;
-        const int i = min_i(st4::kIlevTail - 1, fint(xk));
-        const float delk1 = min_r(1.0f, xk - static_cast<float>(i));
-        const float delk2 = 1.0f - delk1;
-        tau1 = ((f.tauhft2_at(ind, j, i) * deli2 + f.tauhft2_at(ind + 1, j, i) * deli1) * delj2 +
-                (f.tauhft2_at(ind, j + 1, i) * deli2 + f.tauhft2_at(ind + 1, j + 1, i) * deli1) *
-                    delj1) * delk2 +
-               ((f.tauhft2_at(ind, j, i + 1) * deli2 + f.tauhft2_at(ind + 1, j, i + 1) * deli1) *
-                    delj2 +
-                (f.tauhft2_at(ind, j + 1, i + 1) * deli2 +
-                 f.tauhft2_at(ind + 1, j + 1, i + 1) * deli1) *
-                    delj1) *
-                   delk1;
-      } else {
-        tau1 = (f.tauhft_at(ind, j) * deli2 + f.tauhft_at(ind + 1, j) * deli1) * delj2 +
-               (f.tauhft_at(ind, j + 1) * deli2 + f.tauhft_at(ind + 1, j + 1) * deli1) * delj1;
+      c.syncwarp();
+    }
+WWB_UNROLL(1)
+    for (int j = c.lane(); j < l.n; j += Grp::kLanes) {
+      one_copy();
+      const int k = l.at(j);
+      SrceSh& s = x.sh[k];
+      float tauhf = s.tauhf;
+      if (p.sintailpar[0] < 0.5f) tauhf = sum4(x.tr(k) + at.zb, kJtot, 0.0f);
+      float cp, sp;
+      sincosf_i(s.usdirpl, &sp, &cp);
+      float twx = s.stress[0] + tauhf * cp;
+      float twy = s.stress[1] + tauhf * sp;
+      const float tauw = sqrt_f(twx * twx + twy * twy);
+      const float ust2b = max_r(s.r.ustar, kEps2);
+      const float ust2 = ust2b * ust2b;
+      const float tauwb = min_r(tauw, max_r(ust2 - kEps1, kEps2Sq));
+      if (tauwb < tauw) {
+        twx = twx * tauwb / tauw;
+        twy = twy * tauwb / tauw;
       }
-      tauhf = levtail0 * (ust3 * ust3) * tau1;
+      s.tauwx = twx;
+      s.tauwy = twy;
     }
-    float cp, sp;
-    dm::sincosf(usdirpl, &sp, &cp);
-    float twx = xstress + tauhf * cp;
-    float twy = ystress + tauhf * sp;
-    const float tauw = sqrt_f(twx * twx + twy * twy);
-    const float ust2b = max_r(ustar, kEps2);
-    const float ust2 = ust2b * ust2b;
-    const float tauwb = min_r(tauw, max_r(ust2 - kEps1, kEps2Sq));
-    if (tauwb < tauw) {
-      twx = twx * tauwb / tauw;
-      twy = twy * tauwb / tauw;
-    }
-    s.tauwx = twx;
-    s.tauwy = twy;
-  });
+  }
   c.sync();
 }
 
@@ -1026,16 +1255,19 @@ WWB_UNROLL(4)
 /// snl1_rowshift_kernel): VSNL and VDNL. UE, SA1, SA2 of as many slots as fit sit in the transient
 /// region; DA1P, DA1M, DA2P, DA2M and DA1C + DA2C in the slot's global scratch (DA1C and DA2C are read
 /// back only at their own bin, so their sum is kept, the same two roundings).
-WWB_PD void srce_dia(const Grp& c, const SrceGroup& x, const SlotList& all) {
+template <class G>
+WWB_PD void srce_dia(const Grp& c, const G& x, const SlotList& all) {
   const SrceLayout& L = *x.L;
   const Snl1Dev& p = *x.n;
-  const int nth = p.nth, nfr = p.nfr, nfrhgh = p.nfrhgh, nfrchg = p.nfrchg;
-  const int nspec = p.nspec, nspecx = p.nspecx, nk = p.nk;
+  const int nth = x.nth(), nfr = p.nfr, nfrhgh = p.nfrhgh, nfrchg = p.nfrchg;
+  const int nspec = L.nspec, nk = L.nk;
   const int A4 = (L.alen + 3) & ~3, U4 = ((nfrhgh + 1) * nth + 3) & ~3;
   const int per = srce_trans_floats(L, x.ns) / L.dia;
   const float dal1 = p.dal1, dal2 = p.dal2, dal3 = p.dal3;
+WWB_UNROLL(1)
   for (int j0 = 0; j0 < all.n; j0 += per) {
     SlotList l;
+WWB_UNROLL(1)
     for (int j = j0; j < all.n && j < j0 + per; ++j) l.add(all.at(j));
     // Position j of a slot in this round picks its part of the region.
     auto ue_of = [&](int k) {
@@ -1054,14 +1286,19 @@ WWB_PD void srce_dia(const Grp& c, const SrceGroup& x, const SlotList& all) {
       ue_of(k)[U4 + 2 * A4 + ik] = kTpiInv / p.sig[ik] * x.s(k, L.cg1)[ik];
     });
     c.sync();
-    each_bin(c, l, nspec, [&](int k, int i) {
+    struct SlotA {
+      float* ue;
+      const float *spec, *conx;
+    };
+    bins(c, l, nspec, [&](int k) {
       float* const ue = ue_of(k);
-      ue[i + nth] = x.s(k, L.spec)[i] / ue[U4 + 2 * A4 + x.row(i)];
-    });
+      return SlotA{ue + nth, x.s(k, L.spec), ue + U4 + 2 * A4};
+    }, [&](const SlotA& s, int i) { s.ue[i] = s.spec[i] / s.conx[x.row(i)]; });
     c.sync();
     each_row(c, l, nth, [&](int k, int col) {
       float* const ue = ue_of(k);
       float t = ue[nfr * nth + col];
+WWB_UNROLL(1)
       for (int r = nfr + 1; r <= nfrhgh; ++r) {
         t = t * p.fachfe;
         ue[r * nth + col] = t;
@@ -1078,121 +1315,269 @@ WWB_PD void srce_dia(const Grp& c, const SrceGroup& x, const SlotList& all) {
       s.cons = p.snlc1 * (1.0f + p.snls1 / xx * (1.0f - p.snls2 * xx) * dm::expf(x2));
     });
     c.sync();
-    each_bin(c, l, nspecx, [&](int k, int isp) {
-      float* const ue = ue_of(k);
-      float* const sa1 = ue + U4;
-      float* const sa2 = sa1 + A4;
-      const int ifr0 = x.row(isp), ith = isp - ifr0 * nth;
-      int cc[8];
+    // The eight wrapped directions of a bin: constant for a thread.
+    struct Cols {
+      int ith, cc[8];
+    };
+    auto cols = [&](int ith) {
+      Cols q;
+      q.ith = ith;
       for (int n = 0; n < 8; ++n) {
         const int v = ith + p.shift[n];
-        cc[n] = v < 0 ? v + nth : (v >= nth ? v - nth : v);
+        q.cc[n] = v < 0 ? v + nth : (v >= nth ? v - nth : v);
       }
-      const int r1 = p.ifrow[0 * nfrchg + ifr0] * nth;
-      const int r2 = p.ifrow[1 * nfrchg + ifr0] * nth;
-      const int r3 = p.ifrow[2 * nfrchg + ifr0] * nth;
-      const int r4 = p.ifrow[3 * nfrchg + ifr0] * nth;
-      const float e00 = ue[isp + nth];
-      const float ep1 = p.awg[0] * ue[r2 + cc[1]] + p.awg[1] * ue[r2 + cc[0]] +
-                        p.awg[2] * ue[r1 + cc[1]] + p.awg[3] * ue[r1 + cc[0]];
-      const float em1 = p.awg[4] * ue[r4 + cc[7]] + p.awg[5] * ue[r4 + cc[6]] +
-                        p.awg[6] * ue[r3 + cc[7]] + p.awg[7] * ue[r3 + cc[6]];
-      const float ep2 = p.awg[0] * ue[r2 + cc[5]] + p.awg[1] * ue[r2 + cc[4]] +
-                        p.awg[2] * ue[r1 + cc[5]] + p.awg[3] * ue[r1 + cc[4]];
-      const float em2 = p.awg[4] * ue[r4 + cc[3]] + p.awg[5] * ue[r4 + cc[2]] +
-                        p.awg[6] * ue[r3 + cc[3]] + p.awg[7] * ue[r3 + cc[2]];
+      return q;
+    };
+    dirs(c, l, nth, nfrchg, cols, [&](const Cols& q, int k, int ifr0) {
+      float* const ue = ue_of(k);
+      const int* const cc = q.cc;
+      const float* const u1 = ue + p.ifrow[0 * nfrchg + ifr0] * nth;
+      const float* const u2 = ue + p.ifrow[1 * nfrchg + ifr0] * nth;
+      const float* const u3 = ue + p.ifrow[2 * nfrchg + ifr0] * nth;
+      const float* const u4 = ue + p.ifrow[3 * nfrchg + ifr0] * nth;
+      const int isp = ifr0 * nth + q.ith, o = isp + nth;
+      const float e00 = ue[o];
+      const float ep1 = p.awg[0] * u2[cc[1]] + p.awg[1] * u2[cc[0]] +
+                        p.awg[2] * u1[cc[1]] + p.awg[3] * u1[cc[0]];
+      const float em1 = p.awg[4] * u4[cc[7]] + p.awg[5] * u4[cc[6]] +
+                        p.awg[6] * u3[cc[7]] + p.awg[7] * u3[cc[6]];
+      const float ep2 = p.awg[0] * u2[cc[5]] + p.awg[1] * u2[cc[4]] +
+                        p.awg[2] * u1[cc[5]] + p.awg[3] * u1[cc[4]];
+      const float em2 = p.awg[4] * u4[cc[3]] + p.awg[5] * u4[cc[2]] +
+                        p.awg[6] * u3[cc[3]] + p.awg[7] * u3[cc[2]];
       const float ca = x.sh[k].cons * p.af11_row[ifr0];
       const float factor = ca * e00;
       const float sa1a = e00 * (ep1 * dal1 + em1 * dal2);
       const float sa1b = sa1a - ep1 * em1 * dal3;
       const float sa2a = e00 * (ep2 * dal1 + em2 * dal2);
       const float sa2b = sa2a - ep2 * em2 * dal3;
-      const int o = isp + nth;
-      sa1[o] = factor * sa1b;
-      sa2[o] = factor * sa2b;
-      float* const da = x.gs(k, L.da);
-      if (isp < nspec) da[4 * A4 + isp] = ca * (sa1a + sa1b) + ca * (sa2a + sa2b);
-      da[o] = factor * (dal1 * e00 - dal3 * em1);
-      da[A4 + o] = factor * (dal2 * e00 - dal3 * ep1);
-      da[2 * A4 + o] = factor * (dal1 * e00 - dal3 * em2);
-      da[3 * A4 + o] = factor * (dal2 * e00 - dal3 * ep2);
+      ue[U4 + o] = factor * sa1b;
+      ue[U4 + A4 + o] = factor * sa2b;
+      float* const da = x.gs(k, L.da) + o;
+      if (isp < nspec) da[4 * A4 - nth] = ca * (sa1a + sa1b) + ca * (sa2a + sa2b);
+      da[0] = factor * (dal1 * e00 - dal3 * em1);
+      da[A4] = factor * (dal2 * e00 - dal3 * ep1);
+      da[2 * A4] = factor * (dal1 * e00 - dal3 * em2);
+      da[3 * A4] = factor * (dal2 * e00 - dal3 * ep2);
     });
     c.sync();
-    each_bin(c, l, nspec, [&](int k, int isp) {
+    dirs(c, l, nth, nk, cols, [&](const Cols& q, int k, int ifr0) {
       const float* const ue = ue_of(k);
-      const float* const sa1 = ue + U4;
-      const float* const sa2 = sa1 + A4;
-      const float* const da1p = x.gs(k, L.da);
-      const float* const da1m = da1p + A4;
-      const float* const da2p = da1m + A4;
-      const float* const da2m = da2p + A4;
-      const int ifr0 = x.row(isp), ith = isp - ifr0 * nth;
-      int cc[8];
-      for (int n = 0; n < 8; ++n) {
-        const int v = ith + p.shift[n];
-        cc[n] = v < 0 ? v + nth : (v >= nth ? v - nth : v);
-      }
-      const int r5 = p.ifrow[4 * nfrchg + ifr0] * nth;
-      const int r6 = p.ifrow[5 * nfrchg + ifr0] * nth;
-      const int r7 = p.ifrow[6 * nfrchg + ifr0] * nth;
-      const int r8 = p.ifrow[7 * nfrchg + ifr0] * nth;
-      const int o = isp + nth;
-      x.gs(k, L.vsnl)[isp] = ue[U4 + 2 * A4 + ifr0] * (-2.0f * (sa1[o] + sa2[o]) +
-                             p.awg[0] * (sa1[r6 + cc[5]] + sa2[r6 + cc[1]]) +
-                             p.awg[1] * (sa1[r6 + cc[4]] + sa2[r6 + cc[0]]) +
-                             p.awg[2] * (sa1[r5 + cc[5]] + sa2[r5 + cc[1]]) +
-                             p.awg[3] * (sa1[r5 + cc[4]] + sa2[r5 + cc[0]]) +
-                             p.awg[4] * (sa1[r8 + cc[3]] + sa2[r8 + cc[7]]) +
-                             p.awg[5] * (sa1[r8 + cc[2]] + sa2[r8 + cc[6]]) +
-                             p.awg[6] * (sa1[r7 + cc[3]] + sa2[r7 + cc[7]]) +
-                             p.awg[7] * (sa1[r7 + cc[2]] + sa2[r7 + cc[6]]));
-      x.gs(k, L.vdnl)[isp] = -2.0f * da1p[4 * A4 + isp] +
-                             p.swg[0] * (da1p[r6 + cc[5]] + da2p[r6 + cc[1]]) +
-                             p.swg[1] * (da1p[r6 + cc[4]] + da2p[r6 + cc[0]]) +
-                             p.swg[2] * (da1p[r5 + cc[5]] + da2p[r5 + cc[1]]) +
-                             p.swg[3] * (da1p[r5 + cc[4]] + da2p[r5 + cc[0]]) +
-                             p.swg[4] * (da1m[r8 + cc[3]] + da2m[r8 + cc[7]]) +
-                             p.swg[5] * (da1m[r8 + cc[2]] + da2m[r8 + cc[6]]) +
-                             p.swg[6] * (da1m[r7 + cc[3]] + da2m[r7 + cc[7]]) +
-                             p.swg[7] * (da1m[r7 + cc[2]] + da2m[r7 + cc[6]]);
+      const float* const sa = ue + U4;
+      const float* const da = x.gs(k, L.da);
+      const int* const cc = q.cc;
+      const int o5 = p.ifrow[4 * nfrchg + ifr0] * nth;
+      const int o6 = p.ifrow[5 * nfrchg + ifr0] * nth;
+      const int o7 = p.ifrow[6 * nfrchg + ifr0] * nth;
+      const int o8 = p.ifrow[7 * nfrchg + ifr0] * nth;
+      const int isp = ifr0 * nth + q.ith, o = isp + nth;
+      // DA*P rows 5, 6 and DA*M rows 7, 8 of the two interactions, all on their way at once.
+      const float *const d5 = da + o5, *const d6 = da + o6, *const d7 = da + A4 + o7,
+                  *const d8 = da + A4 + o8;
+      const float p65 = d6[cc[5]], p64 = d6[cc[4]], p55 = d5[cc[5]], p54 = d5[cc[4]];
+      const float q61 = d6[2 * A4 + cc[1]], q60 = d6[2 * A4 + cc[0]], q51 = d5[2 * A4 + cc[1]],
+                  q50 = d5[2 * A4 + cc[0]];
+      const float m83 = d8[cc[3]], m82 = d8[cc[2]], m73 = d7[cc[3]], m72 = d7[cc[2]];
+      const float n87 = d8[2 * A4 + cc[7]], n86 = d8[2 * A4 + cc[6]], n77 = d7[2 * A4 + cc[7]],
+                  n76 = d7[2 * A4 + cc[6]];
+      const float dc = da[4 * A4 + isp];
+      const float *const s5 = sa + o5, *const s6 = sa + o6, *const s7 = sa + o7, *const s8 = sa + o8;
+      x.gs(k, L.vsnl)[isp] = ue[U4 + 2 * A4 + ifr0] * (-2.0f * (sa[o] + sa[A4 + o]) +
+                             p.awg[0] * (s6[cc[5]] + s6[A4 + cc[1]]) +
+                             p.awg[1] * (s6[cc[4]] + s6[A4 + cc[0]]) +
+                             p.awg[2] * (s5[cc[5]] + s5[A4 + cc[1]]) +
+                             p.awg[3] * (s5[cc[4]] + s5[A4 + cc[0]]) +
+                             p.awg[4] * (s8[cc[3]] + s8[A4 + cc[7]]) +
+                             p.awg[5] * (s8[cc[2]] + s8[A4 + cc[6]]) +
+                             p.awg[6] * (s7[cc[3]] + s7[A4 + cc[7]]) +
+                             p.awg[7] * (s7[cc[2]] + s7[A4 + cc[6]]));
+      x.gs(k, L.vdnl)[isp] = -2.0f * dc + p.swg[0] * (p65 + q61) + p.swg[1] * (p64 + q60) +
+                             p.swg[2] * (p55 + q51) + p.swg[3] * (p54 + q50) +
+                             p.swg[4] * (m83 + n87) + p.swg[5] * (m82 + n86) +
+                             p.swg[6] * (m73 + n77) + p.swg[7] * (m72 + n76);
     });
     c.sync();
   }
 }
 
 // ------------------------------------------------------------------------------------ W3SDS4
-/// The cumulative term's sums over B-wide blocks of one IK2 row for up to kSlots points:
-/// v[j] += sum over the row of CUMULW * BRLAMBDA in order, for the slots of `mask`.
-template <int B>
-WWB_PD void cumul_row(const float* cw, size_t step, const float* const* brl, int nth,
-                      unsigned mask, float* v) {
-  for (int j0 = 0; j0 < nth; j0 += B) {
-    float q[B];
+WWB_PD int first_bit(unsigned m) {
+#if defined(__CUDA_ARCH__)
+  return __ffs(static_cast<int>(m)) - 1;
+#else
+  return __builtin_ctz(m);
+#endif
+}
+
+/// BTH of the saturation (:2262-2290) for up to NS listed slots. A thread takes a bin of every slot, so
+/// the weights and indices are read once for all of them; a missing slot repeats the first one.
+template <int NS, class G>
+WWB_PD void sat_sums(const Grp& c, const G& x, const SlotList& l, int rows, int ik1) {
+  const SrceLayout& L = *x.L;
+  const Fields& f = *x.f;
+  const int nth = x.nth(), nspec = L.nspec, ld = f.sat_ld;
+  const float dth = x.q->dth;
+  const float* spec[NS];
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-    for (int b = 0; b < B; ++b) q[b] = cw[static_cast<size_t>(j0 + b) * step];
+  for (int m = 0; m < NS; ++m) spec[m] = x.s(l.at(m < l.n ? m : 0), L.spec);
+WWB_UNROLL(1)
+  for (int i = c.tid; i < nspec; i += c.nthr) {
+    one_copy();
+    const int ik0 = x.row(i), ith0 = i - ik0 * nth;
+    const int row = ik0 * nth - 1;
+    const float* sw = f.satw_t + ith0;
+    const int* si = f.sati_t + ith0;
+    float v[NS] = {};
+    if (ik0 + 1 >= ik1) {
+WWB_UNROLL(6)
+      for (int j = 0; j < rows; ++j) {
+        const float w = *sw;
+        const int o = row + *si;
+        sw += ld;
+        si += ld;
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-    for (int j = 0; j < kSlots; ++j) {
-      if (!(mask >> j & 1)) continue;
-      float a = v[j];
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-      for (int b = 0; b < B; b += (B >= 4 ? 4 : 1)) {
-        if (B >= 4) {
-          const F4 r = ld4(brl[j] + j0 + b);
-          a = a + q[b] * r.a;
-          a = a + q[b + (B >= 4 ? 1 : 0)] * r.b;
-          a = a + q[b + (B >= 4 ? 2 : 0)] * r.c;
-          a = a + q[b + (B >= 4 ? 3 : 0)] * r.d;
-        } else {
-          a = a + q[b] * brl[j][j0 + b];
-        }
+        for (int m = 0; m < NS; ++m) v[m] = v[m] + w * spec[m][o];
       }
-      v[j] = a;
+    }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int m = 0; m < NS; ++m) {
+      if (m >= l.n) break;
+      const int k = l.at(m);
+      const float kx = x.s(k, L.wn1)[ik0];
+      const float facsat = (f.sig[ik0 + 1] * ((kx * kx) * kx)) * dth;
+      x.tr(k)[i] = ik0 + 1 >= ik1 ? v[m] * facsat : 0.0f;
+    }
+  }
+}
+
+/// Wave-turbulence interaction and the cumulative effect (:2533-2575) for up to NS listed slots; mask_at
+/// and ren_at: the slots' block masks and (SSDSC(3) > 0) renewal sums in the transient region. A thread
+/// takes a bin of every slot: CUMULW's row is read once for all of them and BRLAMBDA is a broadcast. The
+/// sums grow with the frequency: the warps take the bins from the top, forwards and backwards in turn.
+template <int NS, class G>
+WWB_PD void sds4_turb(const Grp& c, const G& x, const SlotList& l, bool blocks, int dikcumul, int ik1,
+                      int mask_at, int ren_at) {
+  constexpr int NTH = G::kNth;
+  const SrceLayout& L = *x.L;
+  const Fields& f = *x.f;
+  const float* ssdsc = x.q->ssdsc;
+  const int nk = L.nk, nth = x.nth(), nspec = L.nspec;
+  const float sc2 = ssdsc[2], dvc = ssdsc[20] * 4.0f;
+  const float* brl[NS];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int j = 0; j < NS; ++j) brl[j] = x.tr(l.at(j < l.n ? j : 0));
+  const int nch = (nspec + Grp::kLanes - 1) / Grp::kLanes, nw = c.nwarp();
+WWB_UNROLL(1)
+  for (int round = 0; round * nw < nch; ++round) {
+    const int e = nch - 1 - (round * nw + (round & 1 ? nw - 1 - c.warp() : c.warp()));
+    const int i = e * Grp::kLanes + c.lane();
+    if (e < 0 || i >= nspec) continue;
+    one_copy();
+    const int ik0 = x.row(i), ik = ik0 + 1, ith0 = i - ik0 * nth;
+    if (ik < ik1) continue;
+    float ren[NS] = {};
+    if (sc2 < 0.0f) {
+WWB_UNROLL(1)
+      for (int ik2 = ik1; ik2 <= ik - dikcumul; ++ik2) {
+        one_copy();
+        unsigned m[NS], any = 0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int j = 0; j < NS; ++j) {
+          m[j] = j < l.n ? reinterpret_cast<const unsigned*>(brl[j] + mask_at)[ik2 - 1] : 0u;
+          any |= m[j];
+        }
+        if (any == 0) continue;
+        const int is2 = (ik2 - 1) * nth;
+        float v[NS] = {};
+        // CUMULW(IS2+J, IS) as a function of IK2, IK and J - ITH where the table is one (f.cumt), else
+        // the transposed table: consecutive IS are consecutive in both.
+        if (NTH != 0 && NTH % 12 == 0 && blocks && f.cumt != nullptr) {
+          const float* const cw = f.cumt + ((ik2 - 1) * nk + ik0) * (2 * NTH - 1) + (NTH - 1 - ith0);
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+          for (int b0 = 0; b0 < NTH / 4; b0 += 3) {
+            if ((any >> b0 & 7u) == 0) continue;
+            float q[12];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int d = 0; d < 12; ++d) q[d] = cw[4 * b0 + d];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int b = 0; b < 3; ++b) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+              for (int j = 0; j < NS; ++j) {
+                if (m[j] & (1u << (b0 + b))) {
+                  const F4 r = ld4(brl[j] + is2 + 4 * (b0 + b));
+                  v[j] = v[j] + q[4 * b] * r.a;
+                  v[j] = v[j] + q[4 * b + 1] * r.b;
+                  v[j] = v[j] + q[4 * b + 2] * r.c;
+                  v[j] = v[j] + q[4 * b + 3] * r.d;
+                }
+              }
+            }
+          }
+        } else {
+          const bool toe = f.cumt != nullptr;
+          const float* const cw =
+              toe ? f.cumt + (static_cast<size_t>(ik2 - 1) * nk + ik0) * (2 * nth - 1) + (nth - 1 - ith0)
+                  : f.cumulw + static_cast<size_t>(is2) * f.cumulw_ld + i;
+          const size_t step = toe ? 1 : f.cumulw_ld;
+          const int width = blocks ? 4 : nth;
+WWB_UNROLL(1)
+          for (; any; any &= any - 1u) {
+            const int b = first_bit(any);
+WWB_UNROLL(1)
+            for (int d = width * b; d < width * b + width; ++d) {
+              const float q = cw[static_cast<size_t>(d) * step];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+              for (int j = 0; j < NS; ++j)
+                if (m[j] >> b & 1) v[j] = v[j] + q * brl[j][is2 + d];
+            }
+          }
+        }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int j = 0; j < NS; ++j)
+          if (m[j]) ren[j] = ren[j] + v[j];
+      }
+    }
+    const float sig2 = f.sig[ik] * 2.0f, ecos = f.ecos[ith0], esin = f.esin[ith0];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int j = 0; j < NS; ++j) {
+      if (j >= l.n) break;
+      const int k = l.at(j);
+      const SrceSh& s = x.sh[k];
+      const float kx = x.s(k, L.wn1)[ik0];
+      const float facturb2 = -((sig2 * kx) * s.facturb);
+      const float dvisc = -((dvc * kx) * kx);
+      const float renewalfreq = sc2 > 0.0f ? brl[j][ren_at + ik0] : ren[j];
+      const float coswind = ecos * s.cosus + esin * s.sinus;
+      const float dturb = facturb2 * max_r(coswind, 0.0f);
+      const float diag2 = (sc2 * renewalfreq + dturb) + dvisc;
+      float* const vdds = x.gs(k, L.vdds) + i;
+      float* const vsds = x.gs(k, L.vsds) + i;
+      *vdds = *vdds + diag2;
+      *vsds = *vsds + x.s(k, L.spec)[i] * diag2;
     }
   }
 }
@@ -1200,11 +1585,12 @@ WWB_PD void cumul_row(const float* cw, size_t step, const float* const* brl, int
 /// W3SDS4 (w3src4md.F90:2043-2659) of the listed slots: VSDS, VDDS, WHITECAP. BRLAMBDA stays in the
 /// slot's transient region (BTH before it, in place), the NK arrays behind it. The libmvec loops
 /// (:2315, :2500, :2509) use scalar powf/expf in every lane.
-WWB_PD void srce_sds4(const Grp& c, const SrceGroup& x, const SlotList& l) {
+template <class G>
+WWB_PD void srce_sds4(const Grp& c, const G& x, const SlotList& l) {
   const SrceLayout& L = *x.L;
   const st4::Params& p = *x.q;
   const Fields& f = *x.f;
-  const int nk = L.nk, nth = L.nth, nspec = L.nspec;
+  const int nk = L.nk, nth = x.nth(), nspec = L.nspec;
   const int R = (nspec + 3) & ~3, K = (nk + 3) & ~3;
   const float* ssdsc = p.ssdsc;
   const float zero = 0.0f, one = 1.0f;
@@ -1230,21 +1616,9 @@ WWB_PD void srce_sds4(const Grp& c, const SrceGroup& x, const SlotList& l) {
       // Rows of SATWEIGHTS past nsat_eff are all zero for one and the same bin: adding 0 * A once has
       // the effect of adding it for each of them.
       const int rows = f.nsat_eff < f.nsat ? f.nsat_eff + 1 : f.nsat;
-      each_bin(c, l, nspec, [&](int k, int i) {
-        const int ik0 = x.row(i), ith0 = i - ik0 * nth;
-        float v = zero;
-        if (ik0 + 1 >= ik1) {
-          const float* const a = x.s(k, L.spec) + ik0 * nth - 1;
-          const float* const sw = f.satw_t + ith0;
-          const int* const si = f.sati_t + ith0;
-WWB_UNROLL(6)
-          for (int j = 0; j < rows; ++j) v = v + sw[j * f.sat_ld] * a[si[j * f.sat_ld]];
-          const float kx = x.s(k, L.wn1)[ik0];
-          const float facsat = (f.sig[ik0 + 1] * ((kx * kx) * kx)) * dth;
-          v = v * facsat;
-        }
-        brl_of(k)[i] = v;
-      });
+      if (l.n == 1) sat_sums<1>(c, x, l, rows, ik1);
+      else if (l.n == 2) sat_sums<2>(c, x, l, rows, ik1);
+      else sat_sums<kSlots>(c, x, l, rows, ik1);
       c.sync();
     }
     each_row(c, l, nk, [&](int k, int ik0) {
@@ -1261,6 +1635,7 @@ WWB_UNROLL(6)
           float lim = -dm::asfloat(0x7f800000u);
           int i = is0;
           bool found = false;
+WWB_UNROLL(1)
           for (; i < is0 + nth; ++i) {
             if (bth[i] >= lim) {
               lim = bth[i];
@@ -1270,6 +1645,7 @@ WWB_UNROLL(6)
             }
           }
           if (!found) lim = dm::asfloat(0x7fc00000u);
+WWB_UNROLL(1)
           for (; i < is0 + nth; ++i)
             if (bth[i] > lim) lim = bth[i];
           b0 = lim;
@@ -1295,21 +1671,28 @@ WWB_UNROLL(6)
     });
     c.sync();
     const float epsr = sqrt_f(p.ssdsbr);
-    each_bin(c, l, nspec, [&](int k, int i) {
+    struct Slot {
+      float* brl;
+      const float *bth0, *a1, *a2, *a3, *spec;
+      float *vdds, *vsds;
+    };
+    const bool iso = p.ssdsdth >= 180.0f;
+    bins(c, l, nspec, [&](int k) {
+      return Slot{brl_of(k), nka(k, kBth0), nka(k, kA1), nka(k, kA2), nka(k, kA3), x.s(k, L.spec),
+                  x.gs(k, L.vdds), x.gs(k, L.vsds)};
+    }, [&](const Slot& s, int i) {
       const int ik0 = x.row(i);
-      const bool in = ik0 + 1 >= ik1;
       float bth = zero, dd = zero;
-      if (in) {
-        bth = p.ssdsdth >= 180.0f ? nka(k, kBth0)[ik0] : brl_of(k)[i];
-        dd = nka(k, kA2)[ik0] +
-             nka(k, kA3)[ik0] * powf_i(max_r(bth - nka(k, kA1)[ik0], zero), p.ssdsp);
+      if (ik0 + 1 >= ik1) {
+        bth = iso ? s.bth0[ik0] : s.brl[i];
+        dd = s.a2[ik0] + s.a3[ik0] * powf_i(max_r(bth - s.a1[ik0], zero), p.ssdsp);
       }
       const float m = max_r(sqrt_f(bth) - epsr, zero);
       float pbi = m * m;
       pbi = pbi * 28.16f;
-      brl_of(k)[i] = pbi / kTwoPiSq;
-      x.gs(k, L.vdds)[i] = dd;
-      x.gs(k, L.vsds)[i] = dd * x.s(k, L.spec)[i];
+      s.brl[i] = pbi / kTwoPiSq;
+      s.vdds[i] = dd;
+      s.vsds[i] = dd * s.spec[i];
     });
     c.sync();
   } else if (sdscase == 2) {
@@ -1319,6 +1702,7 @@ WWB_UNROLL(6)
       float e = zero, dk = zero;
       if (ik >= ik1) {
         const float* const a = x.s(k, L.spec) + ik0 * nth;
+WWB_UNROLL(1)
         for (int ith = 0; ith < nth; ++ith) e = e + (a[ith] * f.sig[ik]) * dth;
         dk = f.dden[ik0] / ((dth * f.sig[ik]) * x.s(k, L.cg1)[ik0]);
       }
@@ -1345,15 +1729,19 @@ WWB_UNROLL(6)
       if (id > st4::kNdtab) id = st4::kNdtab;
       if (id < 1) id = 1;
       int nkl = 0;
+WWB_UNROLL(1)
       for (int i = 0; i < nk; ++i) hs[i] = efdf[i] = kbar[i] = zero;
+WWB_UNROLL(1)
       for (int ikl = 1; ikl <= nk; ++ikl) {
         iksup[ikl - 1] = f.iktab[(ikl - 1) + (id - 1) * f.iktab_ld];
         if (iksup[ikl - 1] <= nk) {
           float v = zero;
+WWB_UNROLL(1)
           for (int i = ikl; i <= iksup[ikl - 1] - 1; ++i) v = v + e1[i - 1] * dk[i - 1];
           efdf[ikl - 1] = v;
           if (efdf[ikl - 1] != zero) {
             float w = zero;
+WWB_UNROLL(1)
             for (int i = ikl; i <= iksup[ikl - 1] - 1; ++i) w = w + (kk[i - 1] * e1[i - 1]) * dk[i - 1];
             kbar[ikl - 1] = w / efdf[ikl - 1];
           } else {
@@ -1363,7 +1751,9 @@ WWB_UNROLL(6)
           nkl = nkl + 1;
         }
       }
+WWB_UNROLL(1)
       for (int i = 0; i < nk; ++i) dck[i] = qb[i] = zero;
+WWB_UNROLL(1)
       for (int ikl = 1; ikl <= nkl; ++ikl) {
         const float kb = kbar[ikl - 1];
         if (hs[ikl - 1] != zero && kb != zero) {
@@ -1381,19 +1771,25 @@ WWB_UNROLL(6)
           qb[ikl - 1] = zero;
         }
       }
+WWB_UNROLL(1)
       for (int i = 0; i < nk; ++i) {
         s1[i] = s2[i] = zero;
         ntimes[i] = 0;
       }
+WWB_UNROLL(1)
       for (int ikl = 1; ikl <= nkl; ++ikl) {
         if (efdf[ikl - 1] > zero) {
+WWB_UNROLL(1)
           for (int i = ikl; i <= iksup[ikl - 1]; ++i)
             s1[i - 1] = s1[i - 1] + (dck[ikl - 1] * e1[i - 1]) / efdf[ikl - 1];
+WWB_UNROLL(1)
           for (int i = ikl; i <= iksup[ikl - 1]; ++i)
             s2[i - 1] = s2[i - 1] + (qb[ikl - 1] * e1[i - 1]) / efdf[ikl - 1];
+WWB_UNROLL(1)
           for (int i = ikl; i <= iksup[ikl - 1]; ++i) ntimes[i - 1] = ntimes[i - 1] + 1;
         }
       }
+WWB_UNROLL(1)
       for (int i = 0; i < nk; ++i) {
         if (ntimes[i] > 0) {
           s1[i] = s1[i] / static_cast<float>(ntimes[i]);
@@ -1402,6 +1798,7 @@ WWB_UNROLL(6)
           s1[i] = s2[i] = zero;
         }
       }
+WWB_UNROLL(1)
       for (int ik = 1; ik <= nk; ++ik) s1[ik - 1] = s1[ik - 1] / f.sig[ik];
     });
     c.sync();
@@ -1438,6 +1835,7 @@ WWB_UNROLL(6)
         const float cg = x.s(k, L.cg1)[ik0];
         float mssp = zero, msspc2 = zero, mssps2 = zero;
         const float kp = dm::powf(x.s(k, L.wn1)[ik0], ssdsc[19]);
+WWB_UNROLL(1)
         for (int ith = 0; ith < nth; ++ith) {
           const float msslong = ((kp * a[ith]) * f.dden[ik0]) / cg;
           msspc2 = msspc2 + msslong * f.ecos[ith];
@@ -1451,6 +1849,7 @@ WWB_UNROLL(6)
       c.sync();
       each_row(c, l, nk, [&](int k, int i0) {
         float m1 = zero, m3 = zero, m4 = zero;
+WWB_UNROLL(1)
         for (int ik = 0; ik <= i0; ++ik) {
           m1 = m1 + nka(k, kB1)[ik];
           m3 = m3 + nka(k, kB2)[ik];
@@ -1476,6 +1875,7 @@ WWB_UNROLL(6)
       float dirforcum = s.r.dlwmean;
       if (ssdsc[10] > zero) dirforcum = nka(k, kMss2)[ik0];
       float sb = zero;
+WWB_UNROLL(1)
       for (int ith = 0; ith < nth; ++ith)
         sb = sb + max_r((a[ith] * f.sig[ik]) * k3, .00000000000001f) * dth;
       nka(k, kBth0)[ik0] = sb;
@@ -1507,7 +1907,7 @@ WWB_UNROLL(6)
         lmod = one;
       }
       const float c9 = ssdsc[8], c13p1 = ssdsc[12] + one;
-      float b = (((c9 * expf_i(-(p.ssdsbr / bthk))) * nka(k, kB4)[ik0]) / c13p1) * lmod;
+      float b = (((c9 * dm::expf(-(p.ssdsbr / bthk))) * nka(k, kB4)[ik0]) / c13p1) * lmod;
       const float xx = copysignf(b, nka(k, kB5)[ik0]);
       b = xx > zero ? xx : zero;
       brl_of(k)[i] = b;
@@ -1545,12 +1945,37 @@ WWB_UNROLL(6)
         const float pw = dm::powf(nka(k, kBrm12)[ik0] / ssdsc[1], 3.0f / 5.0f);
         const float* const b = brl_of(k) + ik0 * nth;
         float w = zero;
+WWB_UNROLL(1)
         for (int i = 0; i < nth; ++i) w = w + (b[i] * (-ssdsc[1])) * pw;
         c5 = ((((cc * cc) * cc) * w) * p.aairgb / kGrav) * f.dden[ik0] / (f.sig[ik] * cg);
       }
       nka(k, kCoef4)[ik0] = c4;
       nka(k, kCoef5)[ik0] = c5;
     });
+  }
+
+  // Which blocks of four directions of a row the cumulative term has to sum: rows below the breaking
+  // threshold are left out (:2558), and a block whose BRLAMBDA is zero adds +-0 to a sum that starts at
+  // +0, which changes nothing while CUMULW is finite. Rows not made of whole blocks: one bit for all.
+  const bool blocks = (nth & 3) == 0 && nth <= 128 && f.cum_finite;
+  if (ssdsc[2] < zero) {
+    each_row(c, l, nk, [&](int k, int ik0) {
+      unsigned m = 0;
+      if (nka(k, kBth0)[ik0] > p.ssdsbr) {
+        if (blocks) {
+          const float* const b = brl_of(k) + ik0 * nth;
+WWB_UNROLL(1)
+          for (int j = 0; j < nth; j += 4) {
+            const F4 r = ld4(b + j);
+            if (r.a != zero || r.b != zero || r.c != zero || r.d != zero) m |= 1u << (j >> 2);
+          }
+        } else {
+          m = 1;
+        }
+      }
+      reinterpret_cast<unsigned*>(nka(k, kA1))[ik0] = m;
+    });
+    c.sync();
   }
 
   // Wave-turbulence interaction and cumulative effect (:2533-2575).
@@ -1565,6 +1990,7 @@ WWB_UNROLL(6)
       const float cc = f.sig[ik] / kk[ik0];
       float ren = zero;
       if (ik > dikcumul)
+WWB_UNROLL(1)
         for (int ik2 = ik1; ik2 <= ik - dikcumul; ++ik2) {
           const float cc2 = f.sig[ik2] / kk[ik2 - 1];
           const float cumulwiso = ((fabs_f(cc2 - cc) * f.dsip[ik2]) / (cc2 * 0.5f)) * dth;
@@ -1575,75 +2001,9 @@ WWB_UNROLL(6)
     c.sync();
   }
   if (turb) {
-    // Each thread takes a bin of every slot: CUMULW's row is read once for all of them, BRLAMBDA is a
-    // broadcast. The bins of the highest frequencies have the longest sums and come first.
-    const float* brl[kSlots];
-    for (int j = 0; j < kSlots; ++j) brl[j] = brl_of(l.at(j < l.n ? j : 0));
-    const int nch = (nspec + Grp::kLanes - 1) / Grp::kLanes;
-    for (int e = nch - 1 - c.warp(); e >= 0; e -= c.nwarp()) {
-      const int i = e * Grp::kLanes + c.lane();
-      if (i >= nspec) continue;
-      const int ik0 = x.row(i), ik = ik0 + 1, ith0 = i - ik0 * nth;
-      if (ik < ik1) continue;
-      float ren[kSlots] = {0.0f, 0.0f, 0.0f, 0.0f};
-      if (ssdsc[2] < zero && ik > dikcumul) {
-        for (int ik2 = ik1; ik2 <= ik - dikcumul; ++ik2) {
-          unsigned mask = 0;
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-          for (int j = 0; j < kSlots; ++j)
-            if (j < l.n && brl[j][R + kBth0 * K + ik2 - 1] > p.ssdsbr) mask |= 1u << j;
-          if (mask == 0) continue;
-          const int is2 = (ik2 - 1) * nth;
-          const float* row[kSlots];
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-          for (int j = 0; j < kSlots; ++j) row[j] = brl[j] + is2;
-          float v[kSlots] = {0.0f, 0.0f, 0.0f, 0.0f};
-          // CUMULW(IS2+J, IS) as a function of IK2, IK and J - ITH where the table is one (f.cumt), else
-          // the transposed table: consecutive IS are consecutive in both.
-          const float* cw;
-          size_t step;
-          if (f.cumt != nullptr) {
-            const int ld = 2 * nth - 1;
-            cw = f.cumt + (static_cast<size_t>(ik2 - 1) * nk + ik0) * ld + (nth - 1 - ith0);
-            step = 1;
-          } else {
-            cw = f.cumulw + static_cast<size_t>(is2) * f.cumulw_ld + i;
-            step = f.cumulw_ld;
-          }
-          if (nth % 12 == 0) cumul_row<12>(cw, step, row, nth, mask, v);
-          else if (nth % 4 == 0) cumul_row<4>(cw, step, row, nth, mask, v);
-          else cumul_row<1>(cw, step, row, nth, mask, v);
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-          for (int j = 0; j < kSlots; ++j)
-            if (mask >> j & 1) ren[j] = ren[j] + v[j];
-        }
-      }
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-      for (int j = 0; j < kSlots; ++j) {
-        if (j >= l.n) continue;
-        const int k = l.at(j);
-        const SrceSh& s = x.sh[k];
-        const float kx = x.s(k, L.wn1)[ik0];
-        const float facturb2 = -(((f.sig[ik] * 2.0f) * kx) * s.facturb);
-        const float dvisc = -(((ssdsc[20] * 4.0f) * kx) * kx);
-        const float renewalfreq = ssdsc[2] > zero ? nka(k, kRen)[ik0] : ren[j];
-        const float coswind = f.ecos[ith0] * s.cosus + f.esin[ith0] * s.sinus;
-        const float dturb = facturb2 * max_r(coswind, zero);
-        const float diag2 = (ssdsc[2] * renewalfreq + dturb) + dvisc;
-        float* const vdds = x.gs(k, L.vdds) + i;
-        float* const vsds = x.gs(k, L.vsds) + i;
-        *vdds = *vdds + diag2;
-        *vsds = *vsds + x.s(k, L.spec)[i] * diag2;
-      }
-    }
+    if (l.n == 1) sds4_turb<1>(c, x, l, blocks, dikcumul, ik1, R + kA1 * K, R + kRen * K);
+    else if (l.n == 2) sds4_turb<2>(c, x, l, blocks, dikcumul, ik1, R + kA1 * K, R + kRen * K);
+    else sds4_turb<kSlots>(c, x, l, blocks, dikcumul, ik1, R + kA1 * K, R + kRen * K);
   }
   c.sync();
   if (wcap) {
@@ -1656,12 +2016,14 @@ WWB_UNROLL(6)
       const float* const mftk = x.s(k, L.mft);
       float wc0 = zero, wc1 = zero, wc3 = zero;
       if (s.in.flogrd57) {
+WWB_UNROLL(1)
         for (int ik = ik1; ik <= ikc; ++ik) {
           wc0 = wc0 + coef4[ik - 1] * (one - wc0);
           wc3 = wc3 + coef5[ik - 1];
         }
       }
       if (s.in.flogrd58) {
+WWB_UNROLL(1)
         for (int ik = ik1; ik <= nk; ++ik) wc1 = wc1 + coef4[ik - 1] * mftk[ik - 1];
       }
       s.whitecap[0] = wc0;
@@ -1675,10 +2037,11 @@ WWB_UNROLL(6)
 // --------------------------------------------------------------------------------- the step
 /// A step up to the update (:1210-1847) of the listed slots: the step count, W3SLN1, the DIA, W3SDS4,
 /// W3SDB1, W3SBT1, the time step, the new spectrum and the terms of the closing sums.
-WWB_PD void srce_advance(const Grp& c, const SrceGroup& x, const SlotList& l) {
+template <class G>
+WWB_PD void srce_advance(const Grp& c, const G& x, const SlotList& l) {
   const srce::Params& p = *x.p;
   const SrceLayout& L = *x.L;
-  const int nk = L.nk, nth = L.nth, nspec = L.nspec;
+  const int nk = L.nk, nth = x.nth(), nspec = L.nspec;
   const int R = (nspec + 3) & ~3;
   if (p.ln1) {
     // W3SLN1 (w3sln1md.F90:56-211): VSLN = WNF(IK) * DIRF(ITH), formed where it is read.
@@ -1748,6 +2111,7 @@ WWB_PD void srce_advance(const Grp& c, const SrceGroup& x, const SlotList& l) {
       } else if (b < 1.) {
         const double arg = dm::exp_d((q0 - 1.) / bb);
         qb = q0 - bb * (q0 - arg) / (bb - arg);
+WWB_UNROLL(1)
         for (int is = 1; is <= 3; ++is) qb = dm::exp_d((qb - 1.) / bb);
       } else {
         qb = static_cast<double>(1.0f - 0x1p-126f);
@@ -1776,53 +2140,65 @@ WWB_PD void srce_advance(const Grp& c, const SrceGroup& x, const SlotList& l) {
   c.sync();
   // :1484-1533, VS, VD and the MIN over IS of the time step's limit.
   {
-    const int nch = (nspec + Grp::kLanes - 1) / Grp::kLanes, all = l.n * nch;
-    for (int e = c.warp(); e < all; e += c.nwarp()) {
-      const int j = (e >= nch) + (e >= 2 * nch) + (e >= 3 * nch);
-      const int k = l.at(j), i = (e - j * nch) * Grp::kLanes + c.lane();
-      SrceSh& s = x.sh[k];
-      float v = dm::asfloat(0x7f800000u);
-      if (i < s.nspech) {
-        const int ik = x.row(i);
-        const float spec = x.s(k, L.spec)[i];
-        const int nscut = s.nscut;
-        float vdin = x.gs(k, L.vdin)[i];
-        float vsin = vdin * spec;
-        float vsnl = x.gs(k, L.vsnl)[i], vdnl = x.gs(k, L.vdnl)[i];
-        float vsds = x.gs(k, L.vsds)[i], vdds = x.gs(k, L.vdds)[i];
-        float vsln = p.ln1 ? x.s(k, L.wnf)[ik] * x.s(k, L.dirf)[i - ik * nth] : 0.0f;
-        float vdbt = 0.0f, vsbt = 0.0f;
-        if (nscut >= 0) {
-          vdbt = i < nscut ? x.s(k, L.cbeta)[x.g->mapwn[i] - 1] : 0.0f;
-          vsbt = vdbt * spec;
-        }
-        if (s.in.inflags24) {
-          vsnl = s.icescalenl * vsnl;
-          vdnl = s.icescalenl * vdnl;
-          vsln = s.icescaleln * vsln;
-          vsin = s.icescalein * vsin;
-          vdin = s.icescalein * vdin;
-          vsds = s.icescaleds * vsds;
-          vdds = s.icescaleds * vdds;
-        }
-        const float vs = (((vsln + vsin) + vsnl) + vsds) + vsbt;
-        const float vd = ((vdin + vdnl) + vdds) + vdbt;
-        x.gs(k, L.vsds)[i] = vs;
-        x.gs(k, L.vdds)[i] = vd;
-        const float damax =
-            mn(mx(p.xrel * x.gs(k, L.specinit)[i], s.afilt), x.s(k, L.dam)[ik]);
-        const float afac = 1.0f / mx(fabs_f(vs / damax), 1.E-10f);
-        v = afac / mx(mn(vd, 0.0f) * afac + 1.0f, 1.E-10f);
+    struct Slot {
+      const float *spec, *vdin, *vsnl, *vdnl, *specinit, *wnf, *dirf, *cbeta, *dam;
+      float *vsds, *vdds;
+      int nspech, nscut, k;
+      bool ice;
+      float iln, iin, inl, ids, afilt;
+      unsigned low;  ///< bits of the smallest limit so far
+    };
+    struct In {
+      float vdin, vsnl, vdnl, vsds, vdds, specinit;
+    };
+    // The limits are never negative and never NaN (mx and mn take their second operand for
+    // one), so their order is that of their bits.
+    bins_ld<2>(c, l, nspec, [&](int k) {
+      const SrceSh& s = x.sh[k];
+      return Slot{x.s(k, L.spec), x.gs(k, L.vdin), x.gs(k, L.vsnl), x.gs(k, L.vdnl),
+                  x.gs(k, L.specinit), x.s(k, L.wnf), x.s(k, L.dirf), x.s(k, L.cbeta), x.s(k, L.dam),
+                  x.gs(k, L.vsds), x.gs(k, L.vdds), s.nspech, s.nscut, k, s.in.inflags24 != 0,
+                  s.icescaleln, s.icescalein, s.icescalenl, s.icescaleds, s.afilt, 0x7f800000u};
+    }, [&](const Slot& s, int i) {
+      return In{s.vdin[i], s.vsnl[i], s.vdnl[i], s.vsds[i], s.vdds[i], s.specinit[i]};
+    }, [&](Slot& s, int i, const In& in) {
+      if (i >= s.nspech) return;
+      const int ik = x.row(i);
+      const float spec = s.spec[i];
+      float vdin = in.vdin;
+      float vsin = vdin * spec;
+      float vsnl = in.vsnl, vdnl = in.vdnl, vsds = in.vsds, vdds = in.vdds;
+      float vsln = p.ln1 ? s.wnf[ik] * s.dirf[i - ik * nth] : 0.0f;
+      float vdbt = 0.0f, vsbt = 0.0f;
+      if (s.nscut >= 0) {
+        vdbt = i < s.nscut ? s.cbeta[x.g->mapwn[i] - 1] : 0.0f;
+        vsbt = vdbt * spec;
       }
-      // The limits are never negative and never NaN (mx and mn take their second operand for
-      // one), so their order is that of their bits.
+      if (s.ice) {
+        vsnl = s.inl * vsnl;
+        vdnl = s.inl * vdnl;
+        vsln = s.iln * vsln;
+        vsin = s.iin * vsin;
+        vdin = s.iin * vdin;
+        vsds = s.ids * vsds;
+        vdds = s.ids * vdds;
+      }
+      const float vs = (((vsln + vsin) + vsnl) + vsds) + vsbt;
+      const float vd = ((vdin + vdnl) + vdds) + vdbt;
+      s.vsds[i] = vs;
+      s.vdds[i] = vd;
+      const float damax = mn(mx(p.xrel * in.specinit, s.afilt), s.dam[ik]);
+      const float afac = 1.0f / mx(fabs_f(vs / damax), 1.E-10f);
+      const unsigned v = dm::asuint(afac / mx(mn(vd, 0.0f) * afac + 1.0f, 1.E-10f));
+      s.low = v < s.low ? v : s.low;
+    }, [&](const Slot& s) {
 #if defined(__CUDA_ARCH__)
-      const unsigned m = __reduce_min_sync(0xffffffffu, dm::asuint(v));
-      if (c.lane() == 0) atomicMin(&s.vmin, m);
+      const unsigned m = __reduce_min_sync(0xffffffffu, s.low);
+      if (c.lane() == 0) atomicMin(&x.sh[s.k].vmin, m);
 #else
-      if (dm::asuint(v) < s.vmin) s.vmin = dm::asuint(v);
+      if (s.low < x.sh[s.k].vmin) x.sh[s.k].vmin = s.low;
 #endif
-    }
+    });
   }
   c.sync();
   each_chain(c, 0, l, [&](int k) {
@@ -1847,78 +2223,92 @@ WWB_PD void srce_advance(const Grp& c, const SrceGroup& x, const SlotList& l) {
   c.sync();
   // :1761-1847, the update and the terms of the ordered sums (PHIAW and PHIBBL's terms, and whether a
   // bin counts for the wind sea's height).
-  each_bin(c, l, nspec, [&](int k, int i) {
-    const SrceSh& s = x.sh[k];
-    const int ik = x.row(i);
-    const float dt = s.dt, hdt = dt;
-    float* const sp = x.s(k, L.spec) + i;
-    const float spec = *sp;
-    const bool low = i < s.nspech;
-    float vdin = x.gs(k, L.vdin)[i];
-    float vsin = vdin * spec;
-    if (s.in.inflags24 && low) {
-      vsin = s.icescalein * vsin;
-      vdin = s.icescalein * vdin;
-    }
-    float vsdb;
-    if (s.early) {
-      vsdb = x.gs(k, L.vsdb)[i];
-    } else {
-      vsdb = s.vddb * spec;
-      x.gs(k, L.vsdb)[i] = vsdb;
-    }
-    const int nscut = s.nscut;
-    float vdbt = 0.0f, vsbt = 0.0f;
-    if (nscut >= 0) {
-      vdbt = i < nscut ? x.s(k, L.cbeta)[x.g->mapwn[i] - 1] : 0.0f;
-      vsbt = vdbt * spec;
-    }
-    if (low) {
-      const float vs = x.gs(k, L.vsds)[i], vd = x.gs(k, L.vdds)[i];
-      const float einc1 = (dt * vs) / mx(1.0f - hdt * vd, 1.0f);
-      float v;
-      if (s.shave) {
-        const float einc2 = copysignf(mn(fabs_f(einc1), x.s(k, L.dam)[ik]), einc1);
-        v = mx(spec + einc2, 0.0f);
-      } else {
-        v = mx(spec + einc1, 0.0f);
+  {
+    struct Slot {
+      float *spec, *vsdb, *t, *tb;
+      const float *vdin, *vs, *vd, *cbeta, *cg, *dam;
+      unsigned char* wind;
+      int nspech, nscut;
+      bool ice, early, shave;
+      float iin, dt, vddb;
+    };
+    struct In {
+      float vdin, vs, vd;
+    };
+    bins_ld<2>(c, l, nspec, [&](int k) {
+      const SrceSh& s = x.sh[k];
+      float* const t = x.tr(k);
+      return Slot{x.s(k, L.spec), x.gs(k, L.vsdb), t, t + R, x.gs(k, L.vdin), x.gs(k, L.vsds),
+                  x.gs(k, L.vdds), x.s(k, L.cbeta), x.s(k, L.cg1), x.s(k, L.dam),
+                  reinterpret_cast<unsigned char*>(t + 2 * R), s.nspech, s.nscut,
+                  s.in.inflags24 != 0, s.early != 0, s.shave != 0, s.icescalein, s.dt, s.vddb};
+    }, [&](const Slot& s, int i) { return In{s.vdin[i], s.vs[i], s.vd[i]}; },
+    [&](const Slot& s, int i, const In& in) {
+      const int ik = x.row(i);
+      const float dt = s.dt, hdt = dt;
+      const float spec = s.spec[i];
+      const bool low = i < s.nspech;
+      float vdin = in.vdin;
+      float vsin = vdin * spec;
+      if (s.ice && low) {
+        vsin = s.iin * vsin;
+        vdin = s.iin * vdin;
       }
-      const float e2 = (dt * vsdb) / mx(1.0f - hdt * s.vddb, 1.0f);
-      *sp = mx(v + e2, 0.0f);
-    }
-    const float factor = x.g->dden[ik] / x.s(k, L.cg1)[ik];
-    float* const t = x.tr(k);
-    t[i] = ((vsin * dt) * factor) / mx(1.0f - vdin * dt, 1.0f);
-    t[R + i] = ((vsbt * dt) * factor) / mx(1.0f - vdbt * dt, 1.0f);
-    reinterpret_cast<unsigned char*>(t + 2 * R)[i] = vsin > 0.0f ? 1 : 0;
-  });
+      float vsdb;
+      if (s.early) {
+        vsdb = s.vsdb[i];
+      } else {
+        vsdb = s.vddb * spec;
+        s.vsdb[i] = vsdb;
+      }
+      float vdbt = 0.0f, vsbt = 0.0f;
+      if (s.nscut >= 0) {
+        vdbt = i < s.nscut ? s.cbeta[x.g->mapwn[i] - 1] : 0.0f;
+        vsbt = vdbt * spec;
+      }
+      if (low) {
+        const float einc1 = (dt * in.vs) / mx(1.0f - hdt * in.vd, 1.0f);
+        float v;
+        if (s.shave) {
+          const float einc2 = copysignf(mn(fabs_f(einc1), s.dam[ik]), einc1);
+          v = mx(spec + einc2, 0.0f);
+        } else {
+          v = mx(spec + einc1, 0.0f);
+        }
+        const float e2 = (dt * vsdb) / mx(1.0f - hdt * s.vddb, 1.0f);
+        s.spec[i] = mx(v + e2, 0.0f);
+      }
+      const float factor = x.g->dden[ik] / s.cg[ik];
+      s.t[i] = ((vsin * dt) * factor) / mx(1.0f - vdin * dt, 1.0f);
+      s.tb[i] = -(((vsbt * dt) * factor) / mx(1.0f - vdbt * dt, 1.0f));
+      s.wind[i] = vsin > 0.0f ? 1 : 0;
+    }, [](const Slot&) {});
+  }
   c.sync();
 }
 
 /// The closing sums' chains (:1815-1847), roles 4-6.
-WWB_PD void srce_sums(const Grp& c, const SrceGroup& x, const SlotList& l) {
+template <class G>
+WWB_PD void srce_sums(const Grp& c, const G& x, const SlotList& l) {
   const SrceLayout& L = *x.L;
   const int R = (L.nspec + 3) & ~3;
-  each_chain(c, 4, l, [&](int k) {
-    float v = x.sh[k].phiaw;
-    walk4(x.tr(k), L.nspec, [&](float t, int) { v = t + v; });
-    x.sh[k].phiaw = v;
-  });
-  each_chain(c, 5, l, [&](int k) {
-    float v = x.sh[k].phibbl;
-    walk4(x.tr(k) + R, L.nspec, [&](float t, int) { v = v - t; });
-    x.sh[k].phibbl = v;
+  each_chain_of(c, 4, 2, l, [&](int r, int k) {
+    float* const to = r ? &x.sh[k].phibbl : &x.sh[k].phiaw;
+    *to = sum4(x.tr(k) + r * R, L.nspec, *to);  // PHIBBL's terms are stored negated
   });
   each_chain(c, 6, l, [&](int k) {
     // A bin without wind input adds -0, which changes nothing.
     const float* const sp = x.s(k, L.spec);
     const unsigned char* const wind = reinterpret_cast<const unsigned char*>(x.tr(k) + 2 * R);
     float v = 0.0f;
+WWB_UNROLL(1)
     for (int ik = 0; ik < L.nk; ++ik) {
       const float factor = x.g->dden[ik] / x.s(k, L.cg1)[ik];
 WWB_UNROLL(12)
-      for (int i = ik * L.nth; i < (ik + 1) * L.nth; ++i)
-        if (wind[i]) v = v + sp[i] * factor;
+      for (int i = ik * x.nth(); i < (ik + 1) * x.nth(); ++i) {
+        const float t = sp[i] * factor;
+        v = v + (wind[i] ? t : -0.0f);
+      }
     }
     x.sh[k].whitecap[2] = sqrt_f(v) * 4.0f;
   });
@@ -1926,11 +2316,12 @@ WWB_UNROLL(12)
 
 /// After the step's W3SPR4 (:1880-1997): FHIGH, MLIM, SEED, the tail for running slots; SPECINIT and
 /// FHIGH's first value for the slots that end their initialisation (:1122-1179).
-WWB_PD void srce_shape(const Grp& c, const SrceGroup& x, const SlotList& run,
+template <class G>
+WWB_PD void srce_shape(const Grp& c, const G& x, const SlotList& run,
                        const SlotList& fresh2) {
   const srce::Params& p = *x.p;
   const SrceLayout& L = *x.L;
-  const int nk = L.nk, nth = L.nth, nspec = L.nspec;
+  const int nk = L.nk, nth = x.nth(), nspec = L.nspec;
   each_chain(c, 0, run, [&](int k) {
     SrceSh& s = x.sh[k];
     s.fage = p.ffxfa * dm::tanhf((((s.in.u10abs * 0.3f) * s.r.fmeanws) * kTpi) / kGrav);
@@ -1961,6 +2352,7 @@ WWB_PD void srce_shape(const Grp& c, const SrceGroup& x, const SlotList& run,
   c.sync();
   if (run.n == 0) return;
   SlotList lim;
+WWB_UNROLL(1)
   for (int j = 0; j < run.n; ++j)
     if (x.sh[run.at(j)].mlim >= 0.0f) lim.add(run.at(j));
   if (lim.n) {
@@ -1997,6 +2389,7 @@ WWB_PD void srce_shape(const Grp& c, const SrceGroup& x, const SlotList& run,
     if (nkh >= nk) return;
     float* const sp = x.s(k, L.spec) + ith;
     float v = sp[(nkh - 1) * nth];
+WWB_UNROLL(1)
     for (int ik = nkh; ik < nk; ++ik) {
       v = v * p.fachfa + 0.0f;
       sp[ik * nth] = v;
@@ -2006,15 +2399,17 @@ WWB_PD void srce_shape(const Grp& c, const SrceGroup& x, const SlotList& run,
 }
 
 /// 3. After the loop (:2050-2350), FLD2 excepted (ww_srce_init refuses it).
-WWB_PD void srce_finish(const Grp& c, const SrceGroup& x, const SlotList& l) {
+template <class G>
+WWB_PD void srce_finish(const Grp& c, const G& x, const SlotList& l) {
   const srce::Params& p = *x.p;
   const SrceLayout& L = *x.L;
-  const int nk = L.nk, nth = L.nth, nspec = L.nspec;
+  const int nk = L.nk, nth = x.nth(), nspec = L.nspec;
   // Per-IK band sums: eband, a1band, b1band.
   each_row(c, l, nk, [&](int k, int ik) {
     const float* const spec = x.s(k, L.spec);
     const float* const specinit = x.gs(k, L.specinit);
     float eband = 0.0f, a1band = 0.0f, b1band = 0.0f;
+WWB_UNROLL(1)
     for (int ith = 0; ith < nth; ++ith) {
       const float diff = specinit[ith + ik * nth] - spec[ith + ik * nth];
       eband = diff + eband;
@@ -2034,6 +2429,7 @@ WWB_PD void srce_finish(const Grp& c, const SrceGroup& x, const SlotList& l) {
     s.dtdyn = s.dtdyn / static_cast<float>(max_i(s.nsteps, 1));
     s.fcut = s.fhigh * kTpiInv;
     float efinish = 0.0f, mwxfinish = 0.0f, mwyfinish = 0.0f;
+WWB_UNROLL(1)
     for (int ik = 0; ik < nk; ++ik) {
       const float dden = x.g->dden[ik], cg = x.s(k, L.cg1)[ik], wn = x.s(k, L.wn1)[ik];
       efinish = (dden * T[3 * ik]) / cg + efinish;
@@ -2063,9 +2459,11 @@ WWB_PD void srce_finish(const Grp& c, const SrceGroup& x, const SlotList& l) {
     if (s.in.inflags24 && s.in.ice > 0.0f && !p.ic_numerics) {
       s.tauice[0] = s.tauice[1] = 0.0f;
       s.phice = 0.0f;
+WWB_UNROLL(1)
       for (int ik = 0; ik < nk; ++ik) {
         const float factor = x.g->dden[ik] / x.s(k, L.cg1)[ik];
         const float factor2 = ((factor * kGrav) * x.s(k, L.wn1)[ik]) / x.g->sig[ik];
+WWB_UNROLL(1)
         for (int ith = 0; ith < nth; ++ith) {
           const int is = ith + ik * nth;
           const float sp2 = spec[is];
@@ -2180,8 +2578,8 @@ WWB_PD void srce_psc_out(const SrceSh& s, float* psc, float* wc, float* tb, floa
 ///   src.load(c, x, fresh): fills empty slots (SPEC, WN1, CG1, the packets, the state) and lists them
 ///   src.store(c, x, done): writes the finished slots' results out
 /// Both are called by the whole CTA and end with a barrier.
-template <class Src>
-WWB_PD void srce_run(const Grp& c, const SrceGroup& x, Src& src) {
+template <class G, class Src>
+WWB_PD void srce_run(const Grp& c, const G& x, Src& src) {
   const SrceLayout& L = *x.L;
   const int R = (L.nspec + 3) & ~3;
   const int spr4_off = 2 * R + ((((R + 3) / 4) + 3) & ~3);
@@ -2193,6 +2591,7 @@ WWB_PD void srce_run(const Grp& c, const SrceGroup& x, Src& src) {
     src.load(c, x, fresh);
     if (fresh.n) srce_begin(c, x, fresh);
     SlotList all, run, fresh2, wind, done;
+WWB_UNROLL(1)
     for (int k = 0; k < x.ns; ++k) {
       const int st = x.sh[k].state;
       if (st == kIdle) continue;
@@ -2206,6 +2605,7 @@ WWB_PD void srce_run(const Grp& c, const SrceGroup& x, Src& src) {
     // W3SPR4, what follows it, W3SIN4; for SINTAILPAR(4) < 0.5 running slots take W3SPR4 and (unless
     // they end) the next step's W3SIN4 once more. Otherwise the next step's W3SIN4 is this one: it
     // reads the same spectrum, USTAR, Z0 and wind, so it gives the same bits.
+WWB_UNROLL(1)
     for (int rep = 0;; ++rep) {
       const SlotList& spr = rep == 0 ? all : run;
       spr4_sums(c, x, spr, spr4_off);
@@ -2220,12 +2620,14 @@ WWB_PD void srce_run(const Grp& c, const SrceGroup& x, Src& src) {
       });
       if (rep == 0) {
         srce_shape(c, x, run, fresh2);
+WWB_UNROLL(1)
         for (int j = 0; j < run.n; ++j)
           if (x.sh[run.at(j)].done) done.add(run.at(j));
       }
       SlotList next = wind;
       if (rep == 1) {
         next = SlotList();
+WWB_UNROLL(1)
         for (int j = 0; j < run.n; ++j)
           if (!x.sh[run.at(j)].done) next.add(run.at(j));
         c.sync();
@@ -2263,20 +2665,20 @@ struct SrceCtx {
 struct OnePoint {
   SrceIn in;
   bool taken = false;
-  WWB_PD void load(const Grp&, const SrceGroup& x, SlotList& fresh) {
+  WWB_PD void load(const Grp&, const SrceGroup<0>& x, SlotList& fresh) {
     if (taken) return;
     taken = true;
     x.sh[0].in = in;
     x.sh[0].state = in.it != 0 ? kFresh1 : kFresh2;
     fresh.add(0);
   }
-  WWB_PD void store(const Grp&, const SrceGroup& x, const SlotList&) { x.sh[0].state = kIdle; }
+  WWB_PD void store(const Grp&, const SrceGroup<0>& x, const SlotList&) { x.sh[0].state = kIdle; }
 };
 
 /// W3SRCE for one point by one thread (the host build).
 inline void srce_point(const Cta&, const SrceCtx& x) {
   const Grp c{0, 1};
-  const SrceGroup g{x.p, x.g, x.q, x.f, x.n, x.L, x.w, x.gw, x.w + x.L->common + x.L->ws, x.sh, 1};
+  const SrceGroup<0> g{x.p, x.g, x.q, x.f, x.n, x.L, x.w, x.gw, x.w + x.L->common + x.L->ws, x.sh, 1};
   OnePoint src{x.in};
   srce_run(c, g, src);
 }

@@ -10,6 +10,7 @@
 // registrations accepted), :472-584 (init, set, commit status codes).
 #pragma once
 
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -173,6 +174,12 @@ inline std::vector<float> toeplitz_cumulw(const GridReg& g) {
   return t;
 }
 
+inline bool finite_cumulw(const GridReg& g) {
+  for (float v : g.a[A_CUMULW].f)
+    if (!std::isfinite(v)) return false;
+  return true;
+}
+
 /// SATWEIGHTS rows to sum: from the returned row on, every row is zero with the same SATINDICES as
 /// that row (pt::Fields::nsat_eff).
 inline int sat_rows(const GridReg& g) {
@@ -196,6 +203,7 @@ struct FieldPtrs {
       *qbi, *taut, *tauhft, *tauhft2, *fwtable;
   const int *sati_t, *iktab;
   const float* cumt = nullptr;
+  bool cum_finite = false;  ///< every value of the registered CUMULW is finite
   int nsat_eff = -1;  ///< sat_rows of the registration the pointers belong to (-1: every row)
 };
 
@@ -216,6 +224,7 @@ inline pt::Fields make_fields(const GridReg& g, const FieldPtrs& q) {
   f.cumulw = q.cumulw_t;
   f.cumulw_ld = g.a[A_CUMULW].ext[0];
   f.cumt = q.cumt;
+  f.cum_finite = q.cum_finite ? 1 : 0;
   f.nsat_eff = q.nsat_eff < 0 ? f.nsat : q.nsat_eff;
   f.dcki = q.dcki;
   f.qbi = q.qbi;

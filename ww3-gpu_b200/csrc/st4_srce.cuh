@@ -17,7 +17,8 @@ struct St4Dev {
   pt::Fields f;
 };
 
-/// Everything a W3SRCE launch reads besides the per-point arrays (device-resident copy).
+/// Everything a W3SRCE launch reads besides the per-point arrays: a kernel parameter, or (a launch over
+/// several grids) a device-resident copy per grid.
 struct SrceDev {
   srce::Params p;
   pt::SrceGrid g;
@@ -123,9 +124,8 @@ void launch_srce_multi(const SrceJob* jobs_dev, int njobs, int total, const pt::
 /// (work.counter, zeroed here), so points with many substeps do not hold up the rest. Point n's
 /// spectrum is spec + n * nspec, or, with jsea non-null, the resident VA column
 /// spec + jsea[n] * nspec. Per-point packets as ww_srce_batch takes them (device pointers).
-void launch_srce(const SrceDev* d, const pt::SrceLayout& L, SrceStep step, int npts,
-                 float* spec, const int* jsea, const float* wn1, const float* cg1,
-                 const float* pin, float* psc, float* whitecap, float* taubbl, float* tauice,
+void launch_srce(const SrceDev& dev, SrceStep step, int npts, float* spec, const int* jsea,
+                 const float* wn1, const float* cg1, const float* pin, float* psc, float* whitecap, float* taubbl, float* tauice,
                  int* shave, SrceWork& work, cudaStream_t st);
 
 }  // namespace wwb

@@ -97,8 +97,8 @@ struct QueuePoints {
   int total;
   int* counter;
 
-  __device__ __forceinline__ void load(const pt::Grp& c, const pt::SrceGroup& x,
-                                       pt::SlotList& fresh) {
+  template <class G>
+  __device__ __forceinline__ void load(const pt::Grp& c, const G& x, pt::SlotList& fresh) {
     const pt::SrceLayout& L = *x.L;
     if (ctl.empty || ctl.foreign) return;
     bool room = false;
@@ -154,8 +154,8 @@ struct QueuePoints {
     __syncthreads();
   }
 
-  __device__ __forceinline__ void store(const pt::Grp& c, const pt::SrceGroup& x,
-                                        const pt::SlotList& done) {
+  template <class G>
+  __device__ __forceinline__ void store(const pt::Grp& c, const G& x, const pt::SlotList& done) {
     const pt::SrceLayout& L = *x.L;
     const SrceJob& j = ctl.job;
     pt::each_bin(c, done, L.nspec, [&](int k, int i) {
@@ -173,13 +173,37 @@ struct QueuePoints {
   }
 };
 
-/// W3SRCE over the points of one or several grids in one persistent launch: one work queue over
-/// (grid, point), the job of queue entry q the last one whose first entry is <= q. A CTA integrates up
-/// to ns points of one job at a time (srce_point.cuh) and turns to the next job when its slots are
-/// empty. Every job has the same working-set layout (checked on the host).
+/// W3SRCE over the points of one grid. The grid's parameters and table pointers are a kernel parameter,
+/// so the phases read them from the constant bank instead of loading them for every bin.
+template <int NTH>
 __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
-    SrceJob one, const SrceJob* __restrict__ jobs, int njobs, int total, int ns, int* counter,
+    const __grid_constant__ SrceDev dev, const __grid_constant__ SrceJob job, int ns, int* counter,
     float* scratch) {
+  extern __shared__ __align__(16) float w[];
+  __shared__ pt::SrceSh sh[pt::kSlots];
+  __shared__ SrceCtl ctl;
+  const pt::Grp c{static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x)};
+  if (threadIdx.x == 0) {
+    ctl.job = job;
+    ctl.pending = -1;
+    ctl.foreign = ctl.empty = 0;
+    for (int k = 0; k < pt::kSlots; ++k) sh[k].state = pt::kIdle;
+  }
+  __syncthreads();
+  float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
+  const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
+                             w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns};
+  QueuePoints src{ctl, job.npts, counter};
+  pt::srce_run(c, x, src);
+}
+
+/// W3SRCE over the points of several grids in one persistent launch: one work queue over (grid,
+/// point), the job of queue entry q the last one whose first entry is <= q. A CTA integrates points of
+/// one job at a time and turns to the next job when its slots are empty. Every job has the same
+/// working-set layout (checked on the host).
+template <int NTH>
+__global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
+    const SrceJob* __restrict__ jobs, int njobs, int total, int ns, int* counter, float* scratch) {
   extern __shared__ __align__(16) float w[];
   __shared__ pt::SrceSh sh[pt::kSlots];
   __shared__ SrceCtl ctl;
@@ -197,17 +221,13 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
       ctl.foreign = 0;
       ctl.empty = q >= total;
       if (q < total) {
-        if (jobs == nullptr) {
-          ctl.job = one;
-        } else {
-          int lo = 0, hi = njobs - 1;  // the job holding q: first[lo] <= q < first[lo + 1]
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (jobs[mid].first <= q) lo = mid;
-            else hi = mid - 1;
-          }
-          ctl.job = jobs[lo];
+        int lo = 0, hi = njobs - 1;  // the job holding q: first[lo] <= q < first[lo + 1]
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (jobs[mid].first <= q) lo = mid;
+          else hi = mid - 1;
         }
+        ctl.job = jobs[lo];
       }
     }
     __syncthreads();
@@ -220,11 +240,21 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
     }
     __syncthreads();
     float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
-    const pt::SrceGroup x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
-                          w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns};
+    const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
+                               w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns};
     QueuePoints src{ctl, total, counter};
     pt::srce_run(c, x, src);
   }
+}
+
+using OneKernel = void (*)(SrceDev, SrceJob, int, int*, float*);
+using MultiKernel = void (*)(const SrceJob*, int, int, int, int*, float*);
+/// The kernels built for a number of directions: WW3's usual 36 and 24, else the general ones.
+OneKernel one_kernel(int nth) {
+  return nth == 36 ? srce_kernel<36> : nth == 24 ? srce_kernel<24> : srce_kernel<0>;
+}
+MultiKernel multi_kernel(int nth) {
+  return nth == 36 ? srce_multi_kernel<36> : srce_multi_kernel<0>;
 }
 
 /// CTAs per SM of the W3SRCE kernel (0: all that fit), set by the autotuner.
@@ -254,12 +284,14 @@ struct SrcePlan {
   int ns, grid;
   size_t smem;
 };
-int srce_per_sm(const pt::SrceLayout& L, int ns) {
+int srce_per_sm(const pt::SrceLayout& L, int ns, bool multi = false) {
   const size_t smem = srce_smem(L, ns);
-  WWB_CHECK(cudaFuncSetAttribute(srce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const void* const k = multi ? reinterpret_cast<const void*>(multi_kernel(L.nth))
+                              : reinterpret_cast<const void*>(one_kernel(L.nth));
+  WWB_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
   int per_sm = 0;
-  WWB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, srce_kernel, kSrceBlock, smem));
+  WWB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kSrceBlock, smem));
   if (per_sm < 1) throw CudaError(cudaErrorInvalidConfiguration, "srce occupancy");
   return g_srce_ctas_per_sm > 0 && g_srce_ctas_per_sm < per_sm ? g_srce_ctas_per_sm : per_sm;
 }
@@ -272,12 +304,12 @@ int srce_max_slots(const pt::SrceLayout& L) {
 }
 /// One point per CTA until every SM has its CTAs, then more: a launch lasts as long as its longest
 /// point, and a point alone in its CTA is integrated fastest.
-SrcePlan srce_plan(const pt::SrceLayout& L, int npts) {
+SrcePlan srce_plan(const pt::SrceLayout& L, int npts, bool multi = false) {
   if (srce_smem_bytes(L) == 0)
     throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
   const int most = srce_max_slots(L), sms = runtime().sm_count;
   for (int ns = 1;; ++ns) {
-    const long long ctas = static_cast<long long>(srce_per_sm(L, ns)) * sms;
+    const long long ctas = static_cast<long long>(srce_per_sm(L, ns, multi)) * sms;
     if (ns == most || ctas * ns >= npts) {
       const long long want = (static_cast<long long>(npts) + ns - 1) / ns;
       return SrcePlan{ns, static_cast<int>(want < ctas ? want : ctas), srce_smem(L, ns)};
@@ -295,6 +327,12 @@ void srce_reserve_plan(const pt::SrceLayout& L, const SrcePlan& plan, SrceWork& 
     work.scratch_n = need;
   }
 }
+void set_carveout(int nth, int pct) {
+  WWB_CHECK(cudaFuncSetAttribute(reinterpret_cast<const void*>(one_kernel(nth)),
+                                 cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+  WWB_CHECK(cudaFuncSetAttribute(reinterpret_cast<const void*>(multi_kernel(nth)),
+                                 cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+}
 bool srce_reserved(const pt::SrceLayout& L, const SrcePlan& plan, const SrceWork& work) {
   return work.counter != nullptr && static_cast<size_t>(plan.grid) * plan.ns *
                                             static_cast<size_t>(L.total_g) <= work.scratch_n;
@@ -307,8 +345,7 @@ int srce_max_ctas_per_sm(const pt::SrceLayout& L) {
     throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
   const int keep = g_srce_ctas_per_sm;
   g_srce_ctas_per_sm = 0;
-  WWB_CHECK(cudaFuncSetAttribute(srce_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutDefault));
+  set_carveout(L.nth, cudaSharedmemCarveoutDefault);
   const int all = srce_per_sm(L, srce_max_slots(L));
   srce_set_ctas_per_sm(L, keep);  // the carveout of the current choice again
   return all;
@@ -326,7 +363,7 @@ void srce_set_ctas_per_sm(const pt::SrceLayout& L, int ctas) {
     pct = static_cast<int>((100 * ctas * per_cta + 228 * 1024 - 1) / (228 * 1024));
     if (pct > 100) pct = 100;
   }
-  WWB_CHECK(cudaFuncSetAttribute(srce_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+  set_carveout(L.nth, pct);
 }
 
 size_t srce_smem_bytes(const pt::SrceLayout& L) {
@@ -383,35 +420,35 @@ void srce_reserve(const pt::SrceLayout& L, int npts, SrceWork& work, cudaStream_
 }
 
 void srce_multi_reserve(const pt::SrceLayout& L, int total, SrceWork& work) {
-  srce_reserve_plan(L, srce_plan(L, total > 0 ? total : 1), work);
+  srce_reserve_plan(L, srce_plan(L, total > 0 ? total : 1, true), work);
 }
 
 void launch_srce_multi(const SrceJob* jobs_dev, int njobs, int total, const pt::SrceLayout& L,
                        SrceWork& work, cudaStream_t st) {
   if (total <= 0) return;
-  const SrcePlan plan = srce_plan(L, total);
+  const SrcePlan plan = srce_plan(L, total, true);
   if (!srce_reserved(L, plan, work))
     throw CudaError(cudaErrorInvalidValue, "launch_srce_multi: work buffers not reserved");
   WWB_CHECK(cudaMemsetAsync(work.counter, 0, sizeof(int), st));
-  srce_kernel<<<plan.grid, kSrceBlock, plan.smem, st>>>(SrceJob{}, jobs_dev, njobs, total, plan.ns,
-                                                        work.counter, work.scratch);
+  multi_kernel(L.nth)<<<plan.grid, kSrceBlock, plan.smem, st>>>(jobs_dev, njobs, total, plan.ns,
+                                                                work.counter, work.scratch);
   WWB_CHECK(cudaGetLastError());
 }
 
-void launch_srce(const SrceDev* d, const pt::SrceLayout& L, SrceStep step, int npts,
-                 float* spec, const int* jsea, const float* wn1, const float* cg1,
-                 const float* pin, float* psc, float* whitecap, float* taubbl, float* tauice,
+void launch_srce(const SrceDev& dev, SrceStep step, int npts, float* spec, const int* jsea,
+                 const float* wn1, const float* cg1, const float* pin, float* psc, float* whitecap, float* taubbl, float* tauice,
                  int* shave, SrceWork& work, cudaStream_t st) {
   if (npts <= 0) return;
+  const pt::SrceLayout& L = dev.L;
   const SrcePlan plan = srce_plan(L, npts);
   // The work buffers fit after srce_reserve; otherwise (re)allocate them first, after the
   // previous launches on this stream that may still read the old ones.
   srce_reserve(L, npts, work, st);
   WWB_CHECK(cudaMemsetAsync(work.counter, 0, sizeof(int), st));
-  const SrceJob job{d,   step, npts, 0,        spec,   jsea,   wn1,  cg1,
-                    pin, psc,  whitecap, taubbl, tauice, shave};
-  srce_kernel<<<plan.grid, kSrceBlock, plan.smem, st>>>(job, nullptr, 1, npts, plan.ns,
-                                                        work.counter, work.scratch);
+  const SrceJob job{nullptr, step, npts,     0,      spec,   jsea, wn1, cg1,
+                    pin,     psc,  whitecap, taubbl, tauice, shave};
+  one_kernel(L.nth)<<<plan.grid, kSrceBlock, plan.smem, st>>>(dev, job, plan.ns, work.counter,
+                                                              work.scratch);
   WWB_CHECK(cudaGetLastError());
 }
 
