@@ -90,7 +90,7 @@ struct SrceLayout {
   unsigned nth_magic;  ///< i / nth = umulhi(i, nth_magic) for the bins' range
   // shared: what all slots read, then per slot (stride ws), then the transient region
   int pwsig, pwdir, tail, common;
-  int ws, spec, llws, wn1, cg1, dam, pwwn, mft, cbeta, wnf, dirf;
+  int ws, spec, llws, wn1, cg1, dam, pwwn, mft, cbeta, wnf, dirf, jt;  ///< jt: the tail's arrays over its steps
   int tslot;           ///< transient floats a slot needs outside the DIA
   int dia;             ///< transient floats of one slot's DIA
   // global scratch per slot
@@ -139,11 +139,12 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
   L.cbeta = o; o += K;
   L.wnf = o; o += K;
   L.dirf = o; o += r4(nth);
+  L.jt = o; o += 4 * kJtot4;
   L.ws = o - L.common;
   while (L.ws % 32 != 4) L.ws += 4;
   L.tslot = 2 * R + r4((R + 3) / 4) + 8 * K;                  // closing sums + W3SPR4
   if (R + kNkWork * K > L.tslot) L.tslot = R + kNkWork * K;     // W3SDS4
-  const int sin4 = 2 * R + r4((R + 3) / 4) + 8 * K + 4 * kJtot4;
+  const int sin4 = 2 * R + r4((R + 3) / 4) + 8 * K;
   if (sin4 > L.tslot) L.tslot = sin4;
   const int seq = 3 * r4(nth) + 9 * K;
   if (seq > L.tslot) L.tslot = seq;
@@ -169,17 +170,33 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
   return L;
 }
 
-/// A CTA of warps (on the host: one warp of one lane).
+/// The named barriers of a CTA: its working warps' own, and the two over which they hand the tail to the
+/// tail warp and take its results.
+constexpr int kBarWork = 1, kBarTail = 2, kBarTailDone = 3;
+
+/// The working warps of a CTA (on the host: one warp of one lane).
 struct Grp {
   int tid, nthr;
   WWB_PD void sync() const {
 #if defined(__CUDA_ARCH__)
-    __syncthreads();
+    asm volatile("bar.sync %0, %1;" ::"n"(kBarWork), "r"(nthr) : "memory");
 #endif
   }
   WWB_PD void syncwarp() const {
 #if defined(__CUDA_ARCH__)
     __syncwarp();
+#endif
+  }
+  /// All working warps announce to / wait for the tail warp.
+  WWB_PD void tail_go() const {
+#if defined(__CUDA_ARCH__)
+    __threadfence_block();
+    asm volatile("bar.arrive %0, %1;" ::"n"(kBarTail), "r"(nthr + 32) : "memory");
+#endif
+  }
+  WWB_PD void tail_wait() const {
+#if defined(__CUDA_ARCH__)
+    asm volatile("bar.sync %0, %1;" ::"n"(kBarTailDone), "r"(nthr + 32) : "memory");
 #endif
   }
 #if defined(__CUDA_ARCH__)
@@ -207,13 +224,19 @@ WWB_PD void one_copy() {
 
 /// Up to kSlots slot numbers, in registers.
 struct SlotList {
-  int n = 0;
-  unsigned ids = 0;
+  int n;
+  unsigned ids;
   WWB_PD void add(int k) {
     ids |= static_cast<unsigned>(k) << (4 * n);
     ++n;
   }
   WWB_PD int at(int j) const { return (ids >> (4 * j)) & 15; }
+};
+
+/// What the working warps leave for the tail warp.
+struct TailBox {
+  SlotList l;
+  int exit;
 };
 
 /// What the CTA's phases read: the tables of one grid and the slots' memory. NTH: the number of
@@ -232,6 +255,7 @@ struct SrceGroup {
   float* t;    ///< the transient region
   SrceSh* sh;  ///< kSlots of them
   int ns;
+  TailBox* box;  ///< null: the tail runs where it is called
   static constexpr int kNth = NTH;
   WWB_PD int nth() const { return NTH ? NTH : L->nth; }
   WWB_PD float* s(int k, int off) const { return w + off + k * L->ws; }
@@ -761,13 +785,14 @@ WWB_PD bool scan_plain(const st4::Params& p) { return p.ssinthp > 0.0f && p.ssin
 /// Offsets of W3SIN4's NK arrays in a slot's transient region (after the 2 R + R/4 floats of the
 /// stress terms and their signs).
 struct Sin4At {
-  int zcn, cm, const2, cnst, swv, swt, tu, ta, gz, zb, us, lev;
+  int zcn, cm, const2, cnst, swv, swt, tu, ta;
 };
+/// The tail's arrays in a slot's L.jt.
+enum TailAt : int { kGz = 0, kZb = kJtot4, kUs = 2 * kJtot4, kLev = 3 * kJtot4 };
 WWB_PD Sin4At sin4_at(const SrceLayout& L) {
   const int R = (L.nspec + 3) & ~3, K = (L.nk + 3) & ~3;
   const int o = 2 * R + ((((R + 3) / 4) + 3) & ~3);
-  return Sin4At{o, o + K, o + 2 * K, o + 3 * K, o + 4 * K, o + 5 * K, o + 6 * K, o + 7 * K, o + 8 * K,
-                o + 8 * K + kJtot4, o + 8 * K + 2 * kJtot4, o + 8 * K + 3 * kJtot4};
+  return Sin4At{o, o + K, o + 2 * K, o + 3 * K, o + 4 * K, o + 5 * K, o + 6 * K, o + 7 * K};
 }
 
 template <class G>
@@ -908,7 +933,7 @@ WWB_PD float div_by(float a, float b, float y) {
 /// tabulated tail. 50 dependent steps of an exponential, a logarithm, a division and a square root: the
 /// longest chain of a substep, so what does not depend on the step before is taken out of it.
 template <class G>
-WWB_PD void sin4_tail(const G& x, int k, const Sin4At& at) {
+WWB_PD void sin4_tail(const G& x, int k) {
   const SrceLayout& L = *x.L;
   const st4::Params& p = *x.q;
   const Fields& f = *x.f;
@@ -954,7 +979,7 @@ WWB_UNROLL(6)
   s.levtail0 = levtail0;
   if (p.sintailpar[0] < 0.5f) {
     const float* const tt = x.w + L.tail;
-    float* const tr = x.tr(k);
+    float* const tr = x.s(k, L.jt);
     float ustr = ust3;
     const float dely = tt[7 * kJtot];
     float taur = ust3 * ust3;
@@ -966,7 +991,7 @@ WWB_UNROLL(1)
       const float cm = tt[j], cgtail = tt[kJtot + j], rcm = tt[6 * kJtot + j];
       const float zx = div_by(ustr, cm, rcm) + zzalp;
       const float zarg = min_r(kKappa / zx, 20.0f);
-      const float zmu = min_r(tr[at.gz + j] * dm::expf_q(zarg), 1.0f);
+      const float zmu = min_r(tr[kGz + j] * dm::expf_q(zarg), 1.0f);
       const float zlog = min_r(dm::logf_q(zmu), 0.0f);
       const float zlog2 = zlog * zlog;
       const float zbeta = const1 * zmu * (zlog2 * zlog2);
@@ -982,11 +1007,11 @@ WWB_UNROLL(1)
         const float alphat = alpham * tt[5 * kJtot + j] * fm;
         const float th = tt[3 * kJtot + j];
         levtail = levtail0 * 0.5f * (1.0f - th) + p.sintailpar[2] * 0.5f * (1.0f + th) * alphat;
-        tr[at.lev + j] = levtail;
+        tr[kLev + j] = levtail;
       }
       const float us2 = ustr * ustr, w = (j == 0 || j == kJtot - 1) ? 0.5f : 1.0f;
-      tr[at.zb + j] = zbeta;
-      tr[at.us + j] = us2;
+      tr[kZb + j] = zbeta;
+      tr[kUs + j] = us2;
       taur = taur - div_by(w * sp1 * us2 * zbeta * levtail * dely * cgtail, cm, rcm);
       ustr = sqrt_f(max_r(taur, 0.0f));
     }
@@ -1023,6 +1048,57 @@ WWB_UNROLL(1)
   }
 }
 
+/// 3. The tail stress and the stress limit (:799-976) of the listed slots, by one warp: TAUWX and TAUWY.
+template <class G, class Sync>
+WWB_PD void sin4_close(int lane, const G& x, const SlotList& l, Sync syncwarp) {
+  const SrceLayout& L = *x.L;
+  const st4::Params& p = *x.q;
+  {
+WWB_UNROLL(1)
+    for (int j = lane; j < l.n; j += Grp::kLanes) {
+      one_copy();
+      sin4_tail(x, l.at(j));
+    }
+    syncwarp();
+    if (p.sintailpar[0] < 0.5f) {
+      // TAU1's terms: they do not feed the next step of the tail, so they are formed side by side.
+      const float dely = x.w[L.tail + 7 * kJtot];
+WWB_UNROLL(1)
+      for (int e = lane; e < l.n * kJtot; e += Grp::kLanes) {
+        const int n = (e >= kJtot) + (e >= 2 * kJtot) + (e >= 3 * kJtot), k = l.at(n), j = e - n * kJtot;
+        float* const t = x.s(k, L.jt);
+        const float w = (j == 0 || j == kJtot - 1) ? 0.5f : 1.0f;
+        const float lev = p.sintailpar[2] > 0.0f ? t[kLev + j] : x.sh[k].levtail0;
+        t[kZb + j] = w * t[kZb + j] * t[kUs + j] * lev * dely * x.w[L.tail + kJtot + j] /
+                       x.w[L.tail + j];
+      }
+      syncwarp();
+    }
+WWB_UNROLL(1)
+    for (int j = lane; j < l.n; j += Grp::kLanes) {
+      one_copy();
+      const int k = l.at(j);
+      SrceSh& s = x.sh[k];
+      float tauhf = s.tauhf;
+      if (p.sintailpar[0] < 0.5f) tauhf = sum4(x.s(k, L.jt) + kZb, kJtot, 0.0f);
+      float cp, sp;
+      sincosf_i(s.usdirpl, &sp, &cp);
+      float twx = s.stress[0] + tauhf * cp;
+      float twy = s.stress[1] + tauhf * sp;
+      const float tauw = sqrt_f(twx * twx + twy * twy);
+      const float ust2b = max_r(s.r.ustar, kEps2);
+      const float ust2 = ust2b * ust2b;
+      const float tauwb = min_r(tauw, max_r(ust2 - kEps1, kEps2Sq));
+      if (tauwb < tauw) {
+        twx = twx * tauwb / tauw;
+        twy = twy * tauwb / tauw;
+      }
+      s.tauwx = twx;
+      s.tauwy = twy;
+    }
+  }
+}
+
 WWB_PD bool finite_f(float v) { return fabs_f(v) <= 3.402823466e38f; }
 
 /// W3SIN4 (w3src4md.F90:423-1003) of the listed slots with W3SRCE's arguments (:1100, :1239, :2007):
@@ -1054,7 +1130,7 @@ WWB_PD void srce_sin4(const Grp& c, const G& x, const SlotList& l) {
   });
   if (p.sintailpar[0] < 0.5f)
     each_row(c, l, kJtot, [&](int k, int j) {
-      x.tr(k)[at.gz + j] = kGrav * x.sh[k].r.z0 / x.w[L.tail + 4 * kJtot + j];
+      x.s(k, L.jt)[kGz + j] = kGrav * x.sh[k].r.z0 / x.w[L.tail + 4 * kJtot + j];
     });
   c.sync();
   each_chain(c, 0, l, [&](int k) {
@@ -1147,7 +1223,7 @@ WWB_UNROLL(4)
   });
   c.sync();
   // 2. The stress scan over IK (:696-797).
-  SlotList par, ser;
+  SlotList par{}, ser{};
 WWB_UNROLL(1)
   for (int j = 0; j < l.n; ++j) {
     if (x.sh[l.at(j)].scan_par) par.add(l.at(j));
@@ -1202,52 +1278,14 @@ WWB_UNROLL(1)
     scan_serial(c, x, ser, at);
     c.sync();
   }
-  // 3. The tail stress and the stress limit (:799-976), one warp.
-  if (c.role(0)) {
-WWB_UNROLL(1)
-    for (int j = c.lane(); j < l.n; j += Grp::kLanes) {
-      one_copy();
-      sin4_tail(x, l.at(j), at);
-    }
-    c.syncwarp();
-    if (p.sintailpar[0] < 0.5f) {
-      // TAU1's terms: they do not feed the next step of the tail, so they are formed side by side.
-      const float dely = x.w[L.tail + 7 * kJtot];
-WWB_UNROLL(1)
-      for (int e = c.lane(); e < l.n * kJtot; e += Grp::kLanes) {
-        const int n = (e >= kJtot) + (e >= 2 * kJtot) + (e >= 3 * kJtot), k = l.at(n), j = e - n * kJtot;
-        float* const t = x.tr(k);
-        const float w = (j == 0 || j == kJtot - 1) ? 0.5f : 1.0f;
-        const float lev = p.sintailpar[2] > 0.0f ? t[at.lev + j] : x.sh[k].levtail0;
-        t[at.zb + j] = w * t[at.zb + j] * t[at.us + j] * lev * dely * x.w[L.tail + kJtot + j] /
-                       x.w[L.tail + j];
-      }
-      c.syncwarp();
-    }
-WWB_UNROLL(1)
-    for (int j = c.lane(); j < l.n; j += Grp::kLanes) {
-      one_copy();
-      const int k = l.at(j);
-      SrceSh& s = x.sh[k];
-      float tauhf = s.tauhf;
-      if (p.sintailpar[0] < 0.5f) tauhf = sum4(x.tr(k) + at.zb, kJtot, 0.0f);
-      float cp, sp;
-      sincosf_i(s.usdirpl, &sp, &cp);
-      float twx = s.stress[0] + tauhf * cp;
-      float twy = s.stress[1] + tauhf * sp;
-      const float tauw = sqrt_f(twx * twx + twy * twy);
-      const float ust2b = max_r(s.r.ustar, kEps2);
-      const float ust2 = ust2b * ust2b;
-      const float tauwb = min_r(tauw, max_r(ust2 - kEps1, kEps2Sq));
-      if (tauwb < tauw) {
-        twx = twx * tauwb / tauw;
-        twy = twy * tauwb / tauw;
-      }
-      s.tauwx = twx;
-      s.tauwy = twy;
-    }
+  // 3. TAUWX and TAUWY enter the next step's fluxes and W3SPR4 only: the tail warp forms them beside the
+  // next step's DIA and W3SDS4.
+  if (x.box != nullptr) {
+    if (c.tid == 0) x.box->l = l;
+    c.tail_go();
+  } else {
+    sin4_close(0, x, l, [] {});
   }
-  c.sync();
 }
 
 // ------------------------------------------------------------------------- the DIA (W3SNL1)
@@ -1266,7 +1304,7 @@ WWB_PD void srce_dia(const Grp& c, const G& x, const SlotList& all) {
   const float dal1 = p.dal1, dal2 = p.dal2, dal3 = p.dal3;
 WWB_UNROLL(1)
   for (int j0 = 0; j0 < all.n; j0 += per) {
-    SlotList l;
+    SlotList l{};
 WWB_UNROLL(1)
     for (int j = j0; j < all.n && j < j0 + per; ++j) l.add(all.at(j));
     // Position j of a slot in this round picks its part of the region.
@@ -1685,7 +1723,9 @@ WWB_UNROLL(1)
       float bth = zero, dd = zero;
       if (ik0 + 1 >= ik1) {
         bth = iso ? s.bth0[ik0] : s.brl[i];
-        dd = s.a2[ik0] + s.a3[ik0] * powf_i(max_r(bth - s.a1[ik0], zero), p.ssdsp);
+        // Below the threshold the power of 0 is 0 (SSDSP > 0): most warps have no bin above it.
+        const float over = max_r(bth - s.a1[ik0], zero);
+        dd = s.a2[ik0] + s.a3[ik0] * (over == zero && p.ssdsp > zero ? zero : powf_i(over, p.ssdsp));
       }
       const float m = max_r(sqrt_f(bth) - epsr, zero);
       float pbi = m * m;
@@ -2035,10 +2075,16 @@ WWB_UNROLL(1)
 }
 
 // --------------------------------------------------------------------------------- the step
+/// Waits for the tail warp if it was given work.
+WWB_PD void tail_done(const Grp& c, bool& tail) {
+  if (tail) c.tail_wait();
+  tail = false;
+}
+
 /// A step up to the update (:1210-1847) of the listed slots: the step count, W3SLN1, the DIA, W3SDS4,
 /// W3SDB1, W3SBT1, the time step, the new spectrum and the terms of the closing sums.
 template <class G>
-WWB_PD void srce_advance(const Grp& c, const G& x, const SlotList& l) {
+WWB_PD void srce_advance(const Grp& c, const G& x, const SlotList& l, bool& tail) {
   const srce::Params& p = *x.p;
   const SrceLayout& L = *x.L;
   const int nk = L.nk, nth = x.nth(), nspec = L.nspec;
@@ -2201,6 +2247,7 @@ WWB_UNROLL(1)
     });
   }
   c.sync();
+  tail_done(c, tail);
   each_chain(c, 0, l, [&](int k) {
     SrceSh& s = x.sh[k];
     const float dtg = s.in.dtg;
@@ -2304,8 +2351,23 @@ WWB_PD void srce_sums(const Grp& c, const G& x, const SlotList& l) {
 WWB_UNROLL(1)
     for (int ik = 0; ik < L.nk; ++ik) {
       const float factor = x.g->dden[ik] / x.s(k, L.cg1)[ik];
-WWB_UNROLL(12)
-      for (int i = ik * x.nth(); i < (ik + 1) * x.nth(); ++i) {
+      const int nth = x.nth();
+      int i = ik * nth;
+      const int end = i + nth;
+      if ((nth & 3) == 0) {
+WWB_UNROLL(3)
+        for (; i < end; i += 4) {
+          const F4 q = ld4(sp + i);
+          const uint32_t b = *reinterpret_cast<const uint32_t*>(wind + i);
+          const float t0 = q.a * factor, t1 = q.b * factor, t2 = q.c * factor, t3 = q.d * factor;
+          v = v + (b & 0xffu ? t0 : -0.0f);
+          v = v + (b & 0xff00u ? t1 : -0.0f);
+          v = v + (b & 0xff0000u ? t2 : -0.0f);
+          v = v + (b & 0xff000000u ? t3 : -0.0f);
+        }
+      }
+WWB_UNROLL(1)
+      for (; i < end; ++i) {
         const float t = sp[i] * factor;
         v = v + (wind[i] ? t : -0.0f);
       }
@@ -2351,7 +2413,7 @@ WWB_PD void srce_shape(const Grp& c, const G& x, const SlotList& run,
            [&](int k, int i) { x.gs(k, L.specinit)[i] = x.s(k, L.spec)[i]; });
   c.sync();
   if (run.n == 0) return;
-  SlotList lim;
+  SlotList lim{};
 WWB_UNROLL(1)
   for (int j = 0; j < run.n; ++j)
     if (x.sh[run.at(j)].mlim >= 0.0f) lim.add(run.at(j));
@@ -2586,11 +2648,12 @@ WWB_PD void srce_run(const Grp& c, const G& x, Src& src) {
   const bool sin4_at_init = x.q->sintailpar[3] > 0.5f;  // :1100
   const bool spr4_twice = x.q->sintailpar[3] < 0.5f;    // :2012
   srce_common(c, x);
+  bool tail = false;  // the tail warp is at work
   for (;;) {
-    SlotList fresh;
+    SlotList fresh{};
     src.load(c, x, fresh);
     if (fresh.n) srce_begin(c, x, fresh);
-    SlotList all, run, fresh2, wind, done;
+    SlotList all{}, run{}, fresh2{}, wind{}, done{};
 WWB_UNROLL(1)
     for (int k = 0; k < x.ns; ++k) {
       const int st = x.sh[k].state;
@@ -2601,7 +2664,7 @@ WWB_UNROLL(1)
       if (st != kFresh1 || sin4_at_init) wind.add(k);
     }
     if (all.n == 0) break;
-    if (run.n) srce_advance(c, x, run);
+    if (run.n) srce_advance(c, x, run, tail);
     // W3SPR4, what follows it, W3SIN4; for SINTAILPAR(4) < 0.5 running slots take W3SPR4 and (unless
     // they end) the next step's W3SIN4 once more. Otherwise the next step's W3SIN4 is this one: it
     // reads the same spectrum, USTAR, Z0 and wind, so it gives the same bits.
@@ -2610,6 +2673,7 @@ WWB_UNROLL(1)
       const SlotList& spr = rep == 0 ? all : run;
       spr4_sums(c, x, spr, spr4_off);
       c.sync();
+      tail_done(c, tail);
       spr4_chains(c, x, spr, spr4_off);
       if (rep == 0 && run.n) srce_sums(c, x, run);
       c.sync();
@@ -2626,13 +2690,16 @@ WWB_UNROLL(1)
       }
       SlotList next = wind;
       if (rep == 1) {
-        next = SlotList();
+        next = SlotList{};
 WWB_UNROLL(1)
         for (int j = 0; j < run.n; ++j)
           if (!x.sh[run.at(j)].done) next.add(run.at(j));
         c.sync();
       }
-      if (next.n) srce_sin4(c, x, next);
+      if (next.n) {
+        srce_sin4(c, x, next);
+        tail = x.box != nullptr;
+      }
       if (!(rep == 0 && spr4_twice && run.n)) break;
     }
     each_chain(c, 0, all, [&](int k) {
@@ -2641,6 +2708,7 @@ WWB_UNROLL(1)
     });
     c.sync();
     if (done.n) {
+      tail_done(c, tail);
       srce_finish(c, x, done);
       src.store(c, x, done);
     }
@@ -2678,7 +2746,7 @@ struct OnePoint {
 /// W3SRCE for one point by one thread (the host build).
 inline void srce_point(const Cta&, const SrceCtx& x) {
   const Grp c{0, 1};
-  const SrceGroup<0> g{x.p, x.g, x.q, x.f, x.n, x.L, x.w, x.gw, x.w + x.L->common + x.L->ws, x.sh, 1};
+  const SrceGroup<0> g{x.p, x.g, x.q, x.f, x.n, x.L, x.w, x.gw, x.w + x.L->common + x.L->ws, x.sh, 1, nullptr};
   OnePoint src{x.in};
   srce_run(c, g, src);
 }

@@ -37,8 +37,8 @@ struct SrceStep {
 /// Threads of every ST4 CTA (one CTA per point).
 constexpr int kSt4Block = 256;
 
-/// Threads of a W3SRCE CTA, and the CTAs per SM it is built for: one CTA's ordered chains run beside
-/// the other's parallel phases.
+/// Threads of a W3SRCE CTA (the last warp forms the tails), and the CTAs per SM it is built for: one
+/// CTA's ordered chains run beside the other's parallel phases.
 constexpr int kSrceBlock = 384;
 constexpr int kSrceMinBlocks = 2;
 

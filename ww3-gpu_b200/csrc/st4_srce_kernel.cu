@@ -104,7 +104,7 @@ struct QueuePoints {
     bool room = false;
     for (int k = 0; k < x.ns; ++k) room = room || x.sh[k].state == pt::kIdle;
     if (!room) return;
-    __syncthreads();  // every thread has read the states and the queue's
+    c.sync();  // every thread has read the states and the queue's
     if (c.tid == 0) {
       unsigned m = 0;
       for (int k = 0; k < x.ns; ++k) {
@@ -126,7 +126,7 @@ struct QueuePoints {
       }
       ctl.fresh = m;
     }
-    __syncthreads();
+    c.sync();
     const unsigned m = ctl.fresh;
     for (int k = 0; k < x.ns; ++k)
       if (m >> k & 1) fresh.add(k);
@@ -151,7 +151,7 @@ struct QueuePoints {
       s.in = pt::srce_in(j.step.it, j.step.inflags24, j.step.flogrd57, j.step.flogrd58, j.step.dtg,
                          j.pin + n * srce::NPIN);
     });
-    __syncthreads();
+    c.sync();
   }
 
   template <class G>
@@ -169,9 +169,28 @@ struct QueuePoints {
                        j.tauice + 2 * n, j.shave + n);
       x.sh[k].state = pt::kIdle;
     });
-    __syncthreads();
+    c.sync();
   }
 };
+
+/// The last warp of a CTA: the tails the working warps hand over, until they are done.
+template <class G>
+__device__ __forceinline__ void tail_warp(const G& x, pt::TailBox& box) {
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    asm volatile("bar.sync %0, %1;" ::"n"(pt::kBarTail), "n"(kSrceBlock) : "memory");
+    if (box.exit) break;
+    const pt::SlotList l = box.l;
+    pt::sin4_close(lane, x, l, [] { __syncwarp(); });
+    __threadfence_block();
+    asm volatile("bar.arrive %0, %1;" ::"n"(pt::kBarTailDone), "n"(kSrceBlock) : "memory");
+  }
+}
+__device__ __forceinline__ void tail_exit(const pt::Grp& c, pt::TailBox& box) {
+  c.sync();
+  if (c.tid == 0) box.exit = 1;
+  c.tail_go();
+}
 
 /// W3SRCE over the points of one grid. The grid's parameters and table pointers are a kernel parameter,
 /// so the phases read them from the constant bank instead of loading them for every bin.
@@ -182,8 +201,10 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
   extern __shared__ __align__(16) float w[];
   __shared__ pt::SrceSh sh[pt::kSlots];
   __shared__ SrceCtl ctl;
-  const pt::Grp c{static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x)};
+  __shared__ pt::TailBox box;
+  const pt::Grp c{static_cast<int>(threadIdx.x), kSrceBlock - 32};
   if (threadIdx.x == 0) {
+    box.exit = 0;
     ctl.job = job;
     ctl.pending = -1;
     ctl.foreign = ctl.empty = 0;
@@ -192,9 +213,14 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
   __syncthreads();
   float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
   const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
-                             w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns};
+                             w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns, &box};
+  if (threadIdx.x >= kSrceBlock - 32) {
+    tail_warp(x, box);
+    return;
+  }
   QueuePoints src{ctl, job.npts, counter};
   pt::srce_run(c, x, src);
+  tail_exit(c, box);
 }
 
 /// W3SRCE over the points of several grids in one persistent launch: one work queue over (grid,
@@ -208,13 +234,23 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
   __shared__ pt::SrceSh sh[pt::kSlots];
   __shared__ SrceCtl ctl;
   __shared__ SrceDev dev;
-  const pt::Grp c{static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x)};
+  __shared__ pt::TailBox box;
+  const pt::Grp c{static_cast<int>(threadIdx.x), kSrceBlock - 32};
   if (threadIdx.x == 0) {
+    box.exit = 0;
     ctl.pending = -1;
     for (int k = 0; k < pt::kSlots; ++k) sh[k].state = pt::kIdle;
   }
+  __syncthreads();
+  if (threadIdx.x >= kSrceBlock - 32) {
+    // The grid's parameters change only between jobs, when no tail is under way.
+    const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L, w, nullptr,
+                               nullptr, sh, ns, &box};
+    tail_warp(x, box);
+    return;
+  }
   for (;;) {
-    __syncthreads();
+    c.sync();
     if (threadIdx.x == 0) {
       const int q = ctl.pending >= 0 ? ctl.pending : atomicAdd(counter, 1);
       ctl.pending = q;
@@ -230,21 +266,22 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
         ctl.job = jobs[lo];
       }
     }
-    __syncthreads();
+    c.sync();
     if (ctl.empty) break;
     {
       const int* const from = reinterpret_cast<const int*>(ctl.job.d);
       int* const to = reinterpret_cast<int*>(&dev);
-      for (int i = threadIdx.x; i < static_cast<int>(sizeof(SrceDev) / sizeof(int)); i += blockDim.x)
+      for (int i = threadIdx.x; i < static_cast<int>(sizeof(SrceDev) / sizeof(int)); i += c.nthr)
         to[i] = from[i];
     }
-    __syncthreads();
+    c.sync();
     float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
     const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
-                               w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns};
+                               w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns, &box};
     QueuePoints src{ctl, total, counter};
     pt::srce_run(c, x, src);
   }
+  tail_exit(c, box);
 }
 
 using OneKernel = void (*)(SrceDev, SrceJob, int, int*, float*);
@@ -277,7 +314,7 @@ size_t srce_smem(const pt::SrceLayout& L, int ns) {
   return static_cast<size_t>(pt::srce_shared_floats(L, ns)) * sizeof(float);
 }
 constexpr size_t kSrceStatic =
-    sizeof(pt::SrceSh) * pt::kSlots + sizeof(SrceCtl) + sizeof(SrceDev) + 64;
+    sizeof(pt::SrceSh) * pt::kSlots + sizeof(SrceCtl) + sizeof(SrceDev) + sizeof(pt::TailBox) + 64;
 
 /// A W3SRCE launch: slots per CTA, CTAs, shared memory.
 struct SrcePlan {
