@@ -61,7 +61,7 @@ struct GridCtx {
   DevVec<int> sati_t;
   DevVec<float> cumulw_t;
   DevVec<float> cumt;               ///< CUMULW by (IK2, IK, J - ITH), where it is a function of those
-  bool has_cumt = false, cum_finite = false;
+  bool has_cumt = false, trig_rows = false, cum_finite = false;
   int nsat_eff = -1;                ///< SATWEIGHTS rows to sum
   St4Dev host{};                    ///< the kernel parameters (module state of the commit)
   St4Dev* dev = nullptr;            ///< their device copy
@@ -95,7 +95,7 @@ void refresh(GridCtx& g) {
                    g.cumulw_t.ptr, g.f[st4::A_DCKI].ptr, g.f[st4::A_QBI].ptr,
                    m.f[st4::A_TAUT].ptr,  m.f[st4::A_TAUHFT].ptr, m.f[st4::A_TAUHFT2].ptr,
                    m.f[st4::A_FWTABLE].ptr, g.sati_t.ptr,         g.i[st4::A_IKTAB].ptr,
-                   g.has_cumt ? g.cumt.ptr : nullptr, g.cum_finite, g.nsat_eff};
+                   g.has_cumt ? g.cumt.ptr : nullptr, g.trig_rows, g.cum_finite, g.nsat_eff};
   (void)a;
   g.host.p = st4::current_params(g.reg, m.reg);
   g.host.f = st4::make_fields(g.reg, q);
@@ -445,6 +445,7 @@ int ww_st4_commit(int igrid) {
     const std::vector<float> cumt = st4::toeplitz_cumulw(g.reg);
     g.has_cumt = !cumt.empty();
     g.cumt.upload(cumt);
+    g.trig_rows = st4::repeated_trig(g.reg);
     g.cum_finite = st4::finite_cumulw(g.reg);
     g.nsat_eff = st4::sat_rows(g.reg);
     g.f[st4::A_CUMULW].upload({});  // only the transposed copy is read

@@ -425,6 +425,11 @@ WWB_HD float powf_t(float x, float y) {
 #endif
 WWB_HC float powf(float x, float y) { return powf_t<WWB_POWF_FUSE>(x, y); }
 
+/// powf for x normal and positive, 0 < |y| <= 0.5 (so |y log2 x| < 75).
+WWB_HD bool normal_pos(float x) { return asuint(x) - 0x00800000u < 0x7f800000u - 0x00800000u; }
+WWB_HD float powf_core(float x, float y) {
+  return pow_exp2<WWB_POWF_FUSE>((double)y * pow_log2<WWB_POWF_FUSE>(asuint(x)), 0);
+}
 /// powf for x in [2^-7, 2) and 0 < y < 16: x is normal and |y log2 x| < 126, so none of the special
 /// cases arises; the same operations without their branches.
 WWB_HD float powf_mid(float x, float y) {
@@ -530,6 +535,51 @@ WWB_HD void sincosf_t(float y, float* sinp, float* cosp) {
 #define WWB_SINCOSF_FUSE 3
 #endif
 WWB_HC void sincosf(float x, float* s, float* c) { sincosf_t<WWB_SINCOSF_FUSE>(x, s, c); }
+
+/// sincosf for |y| < 120 without a branch. Below pi/4 the reduction gives n = 0 and x itself, so one
+/// path covers both of its small ranges.
+WWB_HD void sincosf_core(float y, float* sinp, float* cosp) {
+  const double x0 = y;
+  const double r = x0 * kHpiInv24;
+  const int n = ((int32_t)r + 0x800000) >> 24;
+  const double x = fma_d(-(double)n, kHpi, x0);
+  const double s = (n & 3) == 0 || (n & 3) == 3 ? 1.0 : -1.0;
+  float fs, fc;
+  sincosf_poly<WWB_SINCOSF_FUSE>(x * s, x * x, (n & 2) != 0, n, &fs, &fc);
+  const bool tiny = abstop12(y) < abstop12(0x1p-12f);
+  *sinp = tiny ? y : fs;
+  *cosp = tiny ? 1.0f : fc;
+}
+static_assert((WWB_SINCOSF_FUSE & 2) != 0, "sincosf_core fuses the reduction");
+
+// ----------------------------------------------------------------------------- division
+/// An approximation of 1 / b within an ulp.
+WWB_HD float rcp_seed(float b) {
+#if defined(__CUDA_ARCH__)
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  return y;
+#else
+  return 1.0f / b;
+#endif
+}
+/// Whether a / b may be formed by div_core: both normal and within 2^+-60, b's mantissa not all ones
+/// (the one divisor whose reciprocal the Newton steps may leave an ulp off).
+WWB_HD bool div_ok(float a, float b) {
+  return (asuint(a) >> 23 & 0xff) - 67u <= 120u && (asuint(b) >> 23 & 0xff) - 67u <= 120u &&
+         (asuint(b) & 0x7fffffu) != 0x7fffffu;
+}
+/// a / b correctly rounded, without a branch, for div_ok operands (or a = +0): two Newton steps make
+/// y = 1 / b correctly rounded, two corrections with the exact remainder the quotient (Markstein 1990,
+/// IBM J. Res. Dev. 34). As long as the division instruction sequence, but several of them overlap.
+WWB_HD float div_core(float a, float b) {
+  float y = rcp_seed(b);
+  y = fma_f(fma_f(-b, y, 1.0f), y, y);
+  y = fma_f(fma_f(-b, y, 1.0f), y, y);
+  float q = a * y;
+  q = fma_f(fma_f(-b, q, a), y, q);
+  return fma_f(fma_f(-b, q, a), y, q);
+}
 
 // ------------------------------------------------------------------------------ expm1f, tanhf
 /// fdlibm expm1f (float, no fused operations).
@@ -821,6 +871,51 @@ WWB_HD float atan2f_t(float y, float x) {
 #define WWB_ATAN2F_KLIM 60
 #endif
 WWB_HC float atan2f(float y, float x) { return atan2f_t<WWB_ATAN2F_KLIM>(y, x); }
+
+/// Whether atan2f_core takes these arguments: div_ok and at most 2^24 apart, so that none of atan2f's
+/// special cases arises.
+WWB_HD bool atan2f_ok(float y, float x) {
+  const int gap = (int)(asuint(y) >> 23 & 0xff) - (int)(asuint(x) >> 23 & 0xff);
+  return div_ok(y, x) && gap <= 24 && gap >= -24;
+}
+/// atan2f without a branch: atanf's interval is selected. *bad is set where the second division is
+/// not div_core's; the result is then wrong.
+WWB_HD float atan2f_core(float y, float x, bool* bad) {
+  const float q = fabsf(div_core(y, x));
+  const uint32_t iq = asuint(q);
+  const bool i0 = iq >= 0x3ee00000u, i1 = iq >= 0x3f300000u, i2 = iq >= 0x3f980000u,
+             i3 = iq >= 0x401c0000u;
+  float num = 2.0f * q - 1.0f, den = 2.0f + q;
+  num = i1 ? q - 1.0f : num;
+  den = i1 ? q + 1.0f : den;
+  num = i2 ? q - 1.5f : num;
+  den = i2 ? 1.0f + 1.5f * q : den;
+  num = i3 ? -1.0f : num;
+  den = i3 ? q : den;
+  *bad = i0 && (asuint(den) & 0x7fffffu) == 0x7fffffu;
+  const float t = i0 ? div_core(num, den) : q;
+  const float z = t * t, w = z * z;
+  const float T0 = asfloat(0x3eaaaaabu), T1 = asfloat(0xbe4ccccdu), T2 = asfloat(0x3e124925u),
+              T3 = asfloat(0xbde38e38u), T4 = asfloat(0x3dba2e6eu), T5 = asfloat(0xbd9d8795u),
+              T6 = asfloat(0x3d886b35u), T7 = asfloat(0xbd6ef16bu), T8 = asfloat(0x3d4bda59u),
+              T9 = asfloat(0xbd15a221u), T10 = asfloat(0x3c8569d7u);
+  const float s1 = z * (T0 + w * (T2 + w * (T4 + w * (T6 + w * (T8 + w * T10)))));
+  const float s2 = w * (T1 + w * (T3 + w * (T5 + w * (T7 + w * T9))));
+  float hi = asfloat(0x3eed6338u), lo = asfloat(0x31ac3769u);
+  hi = i1 ? asfloat(0x3f490fdau) : hi;
+  lo = i1 ? asfloat(0x33222168u) : lo;
+  hi = i2 ? asfloat(0x3f7b985eu) : hi;
+  lo = i2 ? asfloat(0x33140fb4u) : lo;
+  hi = i3 ? asfloat(0x3fc90fdau) : hi;
+  lo = i3 ? asfloat(0x33a22168u) : lo;
+  const float p = t * (s1 + s2);
+  const float a = i0 ? hi - ((p - lo) - t) : t - p;
+  const float pi = asfloat(0x40490fdbu), pi_lo = asfloat(0xb3bbbd2eu);
+  const bool yneg = (asuint(y) >> 31) != 0;
+  const float b = a - pi_lo;
+  const float right = yneg ? -a : a, left = yneg ? b - pi : pi - b;
+  return (asuint(x) >> 31) != 0 ? left : right;
+}
 
 // ----------------------------------------------------------------------------------- log10f
 /// fdlibm log10f over logf.

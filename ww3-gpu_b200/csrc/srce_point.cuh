@@ -87,9 +87,10 @@ struct SrceSh {
 /// Offsets (in floats) of the working set; see the file header.
 struct SrceLayout {
   int nspec, nk, nth;
+  int plain;  ///< SSDSC(1) = 1, TTAUWSHELTER = 0 and no W3_STAB3: SrceGroup's PLAIN form
   unsigned nth_magic;  ///< i / nth = umulhi(i, nth_magic) for the bins' range
   // shared: what all slots read, then per slot (stride ws), then the transient region
-  int pwsig, pwdir, tail, common;
+  int pwsig, pwdir, tail, ec, es, common;
   int ws, spec, llws, wn1, cg1, dam, pwwn, mft, cbeta, wnf, dirf, jt;  ///< jt: the tail's arrays over its steps
   int tslot;           ///< transient floats a slot needs outside the DIA
   int dia;             ///< transient floats of one slot's DIA
@@ -120,11 +121,14 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
   L.nspec = ns;
   L.nk = nk;
   L.nth = nth;
+  L.plain = nint(q.ssdsc[0]) == 1 && q.ttauwshelter == 0.0f && !q.stab3;
   L.nth_magic = static_cast<unsigned>(0x100000000ULL / static_cast<unsigned>(nth)) + 1u;
   int o = 0;
   L.pwsig = o; o += K;
   L.pwdir = o; o += K;
   L.tail = o; o += r4(7 * kJtot + 1);
+  L.ec = o; o += r4(nth);
+  L.es = o; o += r4(nth);
   L.common = o;
   // Per slot; offsets of slot 0, the others ws further on. SPEC rows start on 16 bytes, and ws is
   // 4 floats more than a multiple of 32, so four lanes reading float4s of four slots meet
@@ -171,15 +175,29 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
 }
 
 /// The named barriers of a CTA: its working warps' own, and the two over which they hand the tail to the
-/// tail warp and take its results.
+/// tail warp and take its results. bar.sync and bar.arrive want the warp's lanes together, and nothing
+/// makes the compiler rejoin them before inline assembly, so __syncwarp comes directly before.
 constexpr int kBarWork = 1, kBarTail = 2, kBarTailDone = 3;
+#if defined(__CUDACC__)
+template <int ID>
+__device__ __forceinline__ void barrier_sync(int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(threads) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ void barrier_arrive(int threads) {
+  __threadfence_block();
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "r"(threads) : "memory");
+}
+#endif
 
 /// The working warps of a CTA (on the host: one warp of one lane).
 struct Grp {
   int tid, nthr;
   WWB_PD void sync() const {
 #if defined(__CUDA_ARCH__)
-    asm volatile("bar.sync %0, %1;" ::"n"(kBarWork), "r"(nthr) : "memory");
+    barrier_sync<kBarWork>(nthr);
 #endif
   }
   WWB_PD void syncwarp() const {
@@ -190,13 +208,12 @@ struct Grp {
   /// All working warps announce to / wait for the tail warp.
   WWB_PD void tail_go() const {
 #if defined(__CUDA_ARCH__)
-    __threadfence_block();
-    asm volatile("bar.arrive %0, %1;" ::"n"(kBarTail), "r"(nthr + 32) : "memory");
+    barrier_arrive<kBarTail>(nthr + 32);
 #endif
   }
   WWB_PD void tail_wait() const {
 #if defined(__CUDA_ARCH__)
-    asm volatile("bar.sync %0, %1;" ::"n"(kBarTailDone), "r"(nthr + 32) : "memory");
+    barrier_sync<kBarTailDone>(nthr + 32);
 #endif
   }
 #if defined(__CUDA_ARCH__)
@@ -241,8 +258,9 @@ struct TailBox {
 
 /// What the CTA's phases read: the tables of one grid and the slots' memory. NTH: the number of
 /// directions where the kernel is built for it (bin addresses and the loops over directions are then
-/// compile-time arithmetic), 0 for any.
-template <int NTH>
+/// compile-time arithmetic), 0 for any. PLAIN: SSDSC(1) = 1 and no sheltering, so the other breaking
+/// forms and the serial stress scan take no part of the kernel's registers and instruction cache.
+template <int NTH, bool PLAIN>
 struct SrceGroup {
   const srce::Params* p;
   const SrceGrid* g;
@@ -257,10 +275,15 @@ struct SrceGroup {
   int ns;
   TailBox* box;  ///< null: the tail runs where it is called
   static constexpr int kNth = NTH;
+  static constexpr bool kPlain = PLAIN;
   WWB_PD int nth() const { return NTH ? NTH : L->nth; }
   WWB_PD float* s(int k, int off) const { return w + off + k * L->ws; }
   WWB_PD float* gs(int k, int off) const { return gw + (off + k * L->total_g); }
   WWB_PD float* tr(int k) const { return t + k * L->tslot; }
+  /// ECOS and ESIN of frequency ik: the one row kept in shared memory where every row of the registered
+  /// arrays is the same, so that a chain does not wait for them.
+  WWB_PD const float* ecos(int ik) const { return f->trig_rows ? w + L->ec : f->ecos + ik * nth(); }
+  WWB_PD const float* esin(int ik) const { return f->trig_rows ? w + L->es : f->esin + ik * nth(); }
   WWB_PD unsigned char* llws(int k) const {
     return reinterpret_cast<unsigned char*>(w + L->llws + k * L->ws);
   }
@@ -453,6 +476,30 @@ WWB_UNROLL(1)
   return v;
 }
 
+/// The same for n known when compiled and a multiple of 4: all loads first.
+template <int N>
+WWB_PD float sum_flagged_n(const float* x, const unsigned char* flag, unsigned want, float v) {
+  F4 q[N / 4];
+  uint32_t b[N / 4];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int i = 0; i < N / 4; ++i) {
+    q[i] = ld4(x + 4 * i);
+    b[i] = *reinterpret_cast<const uint32_t*>(flag + 4 * i);
+  }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int i = 0; i < N / 4; ++i) {
+    v = v + ((b[i] & 0xffu) == want ? q[i].a : -0.0f);
+    v = v + ((b[i] >> 8 & 0xffu) == want ? q[i].b : -0.0f);
+    v = v + ((b[i] >> 16 & 0xffu) == want ? q[i].c : -0.0f);
+    v = v + ((b[i] >> 24) == want ? q[i].d : -0.0f);
+  }
+  return v;
+}
+
 WWB_PD float powf_i(float x, float y) { return dm::powf_t<WWB_POWF_FUSE>(x, y); }
 /// Sine and cosine without a call: its results would pass through memory.
 WWB_PD void sincosf_i(float x, float* s, float* c) { dm::sincosf_t<WWB_SINCOSF_FUSE>(x, s, c); }
@@ -465,6 +512,13 @@ WWB_PD void srce_common(const Grp& c, const G& x) {
   const SrceLayout& L = *x.L;
   const st4::Params& q = *x.q;
   const Fields& f = *x.f;
+  if (f.trig_rows) {
+WWB_UNROLL(1)
+    for (int i = c.tid; i < x.nth(); i += c.nthr) {
+      x.w[L.ec + i] = f.ecos[i];
+      x.w[L.es + i] = f.esin[i];
+    }
+  }
 WWB_UNROLL(1)
   for (int ik = c.tid; ik < L.nk; ik += c.nthr) {
     x.w[L.pwsig + ik] = dm::powf(f.sig[ik + 1], 2.0f * q.wwnmeanptail);
@@ -716,13 +770,12 @@ WWB_UNROLL(1)
   each_chain_of(c, 1, 2, l, [&](int comp, int k) {
       const float* const a = x.s(k, L.spec);
       const float* const sf = x.tr(k) + off + 6 * nk;
-      const float* const e = comp ? f.esin : f.ecos;
-      float v = 0.0f;
+        float v = 0.0f;
 WWB_UNROLL(1)
       for (int ik = 0; ik < nk; ++ik) {
         const float sfk = sf[ik];
         const float* const ar = a + ik * nth;
-        const float* const er = e + ik * nth;
+        const float* const er = comp ? x.esin(ik) : x.ecos(ik);
         int i = 0;
         if ((nth & 3) == 0) {
 WWB_UNROLL(3)
@@ -751,34 +804,51 @@ WWB_UNROLL(1)
 struct ScanK {
   float cm, ucn, const2, cnst, zcn, swv, swt, sig2is;
 };
-/// DSTAB and LLWS of one bin (:739-783). `plain`: 0 < SSINTHP < 16, so that COS**SSINTHP (a cosine
-/// between 0.01 and 1) and the exponential need no special case and the bins of a thread overlap.
-template <class S>
-WWB_PD float scan_bin(const st4::Params& p, const S& s, const ScanK& q, bool plain, float ustar,
-                      float ustp, float coswind, int* lw) {
-  const bool up = coswind > 0.01f;
-  const float xx = coswind * q.ucn;
-  const float zarg = kKappa / xx;
-  const float zlog = q.zcn + zarg;
-  const bool grow = up && zlog < 0.0f;
+/// The swell damping's scalars of a point.
+struct Swell {
+  float fwuorb, fu, fud, pturb, pvisc;
+};
+/// DSTAB and LLWS of one bin (:739-783).
+WWB_PD float scan_bin(const st4::Params& p, const Swell& s, const ScanK& q, float ustar, float ustp,
+                      float coswind, int* lw) {
   float dst = 0.0f;
-  if (plain) {
-    const float zl = grow ? zlog : -1.0f, cw = grow ? coswind : 0.5f;
-    const float zlog2 = zl * zl;
-    const float g = q.cnst * dm::expf_neg(zl) * (zlog2 * zlog2) * q.ucn * q.ucn *
-                    dm::powf_mid(cw, p.ssinthp);
-    dst = grow ? g : 0.0f;
-  } else if (grow) {
-    const float zlog2 = zlog * zlog;
-    dst = q.cnst * dm::expf(zlog) * (zlog2 * zlog2) * q.ucn * q.ucn * dm::powf(coswind, p.ssinthp);
+  int l = 0;
+  if (coswind > 0.01f) {
+    const float zarg = kKappa / (coswind * q.ucn);
+    const float zlog = q.zcn + zarg;
+    if (zlog < 0.0f) {
+      const float zlog2 = zlog * zlog;
+      dst = q.cnst * dm::expf(zlog) * (zlog2 * zlog2) * q.ucn * q.ucn * dm::powf(coswind, p.ssinthp);
+      l = 1;
+    }
+    if (28.0f * q.cm * ustar * coswind >= 1.0f) l = 1;
   }
-  *lw = grow || (up && 28.0f * q.cm * ustar * coswind >= 1.0f) ? 1 : 0;
+  *lw = l;
   if ((p.sswellf[0] != 0.0f && dst < 1E-7f * q.sig2is) || p.sswellf[2] > 0.0f) {
     const float dvisc = q.swv;
     const float dturb = q.swt * (s.fwuorb + (s.fu + s.fud * coswind) * ustp);
     dst = dst + s.pturb * dturb + s.pvisc * dvisc;
   }
   return dst;
+}
+/// The same without a branch, so that the bins of a thread overlap: 0 < SSINTHP < 16 (a cosine between
+/// 0.01 and 1 to that power has no special case); *ok is cleared where the division is not div_core's.
+WWB_PD float scan_bin_q(const st4::Params& p, const Swell& s, const ScanK& q, float ustar, float ustp,
+                        float coswind, int* lw, bool* ok) {
+  const bool up = coswind > 0.01f;
+  const float xx = up ? coswind * q.ucn : 1.0f;
+  *ok = *ok && dm::div_ok(kKappa, xx);
+  const float zlog = q.zcn + dm::div_core(kKappa, xx);
+  const bool grow = up && zlog < 0.0f;
+  const float zl = grow ? zlog : -1.0f, cw = grow ? coswind : 0.5f;
+  const float zlog2 = zl * zl;
+  const float g = q.cnst * dm::expf_neg(zl) * (zlog2 * zlog2) * q.ucn * q.ucn *
+                  dm::powf_mid(cw, p.ssinthp);
+  float dst = grow ? g : 0.0f;
+  *lw = grow || (up && 28.0f * q.cm * ustar * coswind >= 1.0f) ? 1 : 0;
+  const float dturb = q.swt * (s.fwuorb + (s.fu + s.fud * coswind) * ustp);
+  const float damped = dst + s.pturb * dturb + s.pvisc * q.swv;
+  return (p.sswellf[0] != 0.0f && dst < 1E-7f * q.sig2is) || p.sswellf[2] > 0.0f ? damped : dst;
 }
 WWB_PD bool scan_plain(const st4::Params& p) { return p.ssinthp > 0.0f && p.ssinthp < 16.0f; }
 
@@ -844,9 +914,6 @@ WWB_UNROLL(1)
     const float* const a = x.s(k, L.spec);
     unsigned char* const llws = x.llws(k);
     float* const vdin = x.gs(k, L.vdin);
-    struct Swell {
-      float fwuorb, fu, fud, pturb, pvisc;
-    };
     const Swell sw{s.fwuorb, s.fu, s.fud, s.pturb, s.pvisc};
     const float ustar = s.r.ustar, shelter = fabs_f(p.ttauwshelter);
     float ust = ustar, taux = 0.0f, tauy = 0.0f, cosu = 0.0f, sinu = 0.0f, ustp = 0.0f;
@@ -864,36 +931,70 @@ WWB_UNROLL(1)
 WWB_UNROLL(1)
       for (int ik = 0; ik < nk; ++ik) {
         if (on) {
+          const ScanK q0 = scan_k(x, at, t, ik, 0.0f);  // UCN needs USTP, below
           const float taupx = taux - shelter * s.sums[0];
           const float taupy = tauy - shelter * s.sums[1];
-          ustp = min_r(powf_i((taupx * taupx + taupy * taupy), 0.25f), max_r(ust, 0.3f));
-          const float usdirp = dm::atan2f_t<WWB_ATAN2F_KLIM>(taupy, taupx);
-          sincosf_i(usdirp, &sinu, &cosu);
-          const ScanK q = scan_k(x, at, t, ik, ustp);
-WWB_UNROLL(3)
-          for (int ith = sub; ith < nth; ith += kScanLanes) {
-            const int i = ik * nth + ith;
-            const float ecos = f.ecos[i], esin = f.esin[i];
-            const float coswind = (ecos * cosu + esin * sinu);
-            int lw;
-            const float dst = scan_bin(p, sw, q, plain, ustar, ustp, coswind, &lw);
-            if (istab == 2) {
-              vdin[i] = 0.5f * (vdin[i] + dst);
-            } else {
-              vdin[i] = dst;
+          const float tau2 = taupx * taupx + taupy * taupy;
+          float root;
+          bool bad = true;
+          if (dm::normal_pos(tau2) && dm::atan2f_ok(taupy, taupx)) {
+            // One block, so the power and the angle overlap.
+            root = dm::powf_core(tau2, 0.25f);
+            dm::sincosf_core(dm::atan2f_core(taupy, taupx, &bad), &sinu, &cosu);
+          }
+          if (bad) {
+            root = dm::powf(tau2, 0.25f);
+            dm::sincosf(dm::atan2f(taupy, taupx), &sinu, &cosu);
+          }
+          ustp = min_r(root, max_r(ust, 0.3f));
+          ScanK q = q0;
+          q.ucn = ustp * q.cm + p.zzalp;
+          // Rounds of kRound directions a lane, each a block without branches.
+          constexpr int kRound = G::kNth != 0 && G::kNth % kScanLanes == 0 && G::kNth / kScanLanes <= 4
+                                     ? G::kNth / kScanLanes : 1;
+WWB_UNROLL(1)
+          for (int ith = sub; ith < nth; ith += kRound * kScanLanes) {
+            one_copy();
+            float dst[kRound], cw[kRound], ec[kRound], es[kRound];
+            int lw[kRound];
+            bool ok = plain;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int r = 0; r < kRound; ++r) {
+              const int d = ith + r * kScanLanes;
+              ec[r] = x.ecos(ik)[d];
+              es[r] = x.esin(ik)[d];
+              cw[r] = (ec[r] * cosu + es[r] * sinu);
+              dst[r] = scan_bin_q(p, sw, q, ustar, ustp, cw[r], &lw[r], &ok);
             }
-            llws[i] = static_cast<unsigned char>(lw);
-            const float temp2 = q.const2 * dst * a[i];
-            bx[ith] = temp2 * ecos;
-            by[ith] = temp2 * esin;
-            neg[ith] = dst < 0.0f ? 1 : 0;
+            if (!ok) {
+WWB_UNROLL(1)
+              for (int r = 0; r < kRound; ++r) dst[r] = scan_bin(p, sw, q, ustar, ustp, cw[r], &lw[r]);
+            }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int r = 0; r < kRound; ++r) {
+              const int d = ith + r * kScanLanes, i = ik * nth + d;
+              const float temp2 = q.const2 * dst[r] * a[i];
+              bx[d] = temp2 * ec[r];
+              by[d] = temp2 * es[r];
+              neg[d] = dst[r] < 0.0f ? 1 : 0;
+              vdin[i] = istab == 2 ? 0.5f * (vdin[i] + dst[r]) : dst[r];
+              llws[i] = static_cast<unsigned char>(lw[r]);
+            }
           }
         }
         c.syncwarp();
         if (on)
 WWB_UNROLL(1)
           for (int q = sub; q < 4; q += kScanLanes) {
-            s.sums[q] = sum_flagged((q & 1) ? by : bx, neg, nth, static_cast<unsigned>(q >> 1), s.sums[q]);
+            const float* const b = (q & 1) ? by : bx;
+            const unsigned want = static_cast<unsigned>(q >> 1);
+            s.sums[q] = G::kNth != 0 && G::kNth % 4 == 0
+                            ? sum_flagged_n<(G::kNth != 0 ? G::kNth : 4)>(b, neg, want, s.sums[q])
+                            : sum_flagged(b, neg, nth, want, s.sums[q]);
           }
         c.syncwarp();
       }
@@ -914,6 +1015,12 @@ WWB_UNROLL(1)
       s.ustp = ustp;
     }
   }
+}
+
+/// scan_serial out of line, for the rare slot that needs it in a kernel without sheltering.
+template <class G>
+WWB_PN void scan_serial_call(Grp c, G x, SlotList l, Sin4At at) {
+  scan_serial(c, x, l, at);
 }
 
 /// a / b for b in [2^-20, 2^20], correctly rounded, from y = 1 / b correctly rounded (0: unknown): two steps q + (a - b q) y with fused
@@ -967,7 +1074,7 @@ WWB_PD void sin4_tail(const G& x, int k) {
   float temp = 0.0f;
   {
     const float cosu = s.cosu, sinu = s.sinu;
-    const float *const ec = f.ecos + (nk - 1) * nth, *const es = f.esin + (nk - 1) * nth;
+    const float *const ec = x.ecos(nk - 1), *const es = x.esin(nk - 1);
 WWB_UNROLL(6)
     for (int i = 0; i < nth; ++i) {
       const float coswind = (ec[i] * cosu + es[i] * sinu);
@@ -1237,20 +1344,24 @@ WWB_UNROLL(1)
       float *vdin, *t;
       const float* tk;
       unsigned char *llws, *neg;
-      float ustar, ustp, cosu, sinu, fwuorb, fu, fud, pturb, pvisc;
+      float ustar, ustp, cosu, sinu;
+      Swell sw;
     };
     bins(c, par, L.nspec, [&](int k) {
       const SrceSh& s = x.sh[k];
       return Slot{x.s(k, L.spec), x.gs(k, L.vdin), x.tr(k), x.tr(k), x.llws(k),
                   reinterpret_cast<unsigned char*>(x.tr(k) + 2 * R), s.r.ustar, s.ustp, s.cosu, s.sinu,
-                  s.fwuorb, s.fu, s.fud, s.pturb, s.pvisc};
+                  Swell{s.fwuorb, s.fu, s.fud, s.pturb, s.pvisc}};
     }, [&](const Slot& s, int i) {
       const int ik = x.row(i);
       const ScanK q = scan_k(x, at, s.tk, ik, s.ustp);
-      const float ecos = f.ecos[i], esin = f.esin[i];
+      const int ith = i - ik * nth;
+      const float ecos = x.ecos(ik)[ith], esin = x.esin(ik)[ith];
       const float coswind = (ecos * s.cosu + esin * s.sinu);
       int lw;
-      const float dst = scan_bin(p, s, q, plain, s.ustar, s.ustp, coswind, &lw);
+      bool ok = plain;
+      float dst = scan_bin_q(p, s.sw, q, s.ustar, s.ustp, coswind, &lw, &ok);
+      if (!ok) dst = scan_bin(p, s.sw, q, s.ustar, s.ustp, coswind, &lw);
       s.vdin[i] = dst;
       s.llws[i] = static_cast<unsigned char>(lw);
       const float temp2 = q.const2 * dst * s.spec[i];
@@ -1275,7 +1386,8 @@ WWB_UNROLL(1)
   }
   if (ser.n) {
     c.sync();
-    scan_serial(c, x, ser, at);
+    if (G::kPlain) scan_serial_call(c, x, ser, at);
+    else scan_serial(c, x, ser, at);
     c.sync();
   }
   // 3. TAUWX and TAUWY enter the next step's fluxes and W3SPR4 only: the tail warp forms them beside the
@@ -1647,7 +1759,7 @@ WWB_PD void srce_sds4(const Grp& c, const G& x, const SlotList& l) {
     s.sinus = sn;
     s.cosus = cs;
   });
-  const int sdscase = nint(ssdsc[0]);
+  const int sdscase = G::kPlain ? 1 : nint(ssdsc[0]);
   if (sdscase == 1) {
     // 2.a.1 Saturation (:2262-2290).
     if (p.ssdsdth < 180.0f) {
@@ -2733,20 +2845,20 @@ struct SrceCtx {
 struct OnePoint {
   SrceIn in;
   bool taken = false;
-  WWB_PD void load(const Grp&, const SrceGroup<0>& x, SlotList& fresh) {
+  WWB_PD void load(const Grp&, const SrceGroup<0, false>& x, SlotList& fresh) {
     if (taken) return;
     taken = true;
     x.sh[0].in = in;
     x.sh[0].state = in.it != 0 ? kFresh1 : kFresh2;
     fresh.add(0);
   }
-  WWB_PD void store(const Grp&, const SrceGroup<0>& x, const SlotList&) { x.sh[0].state = kIdle; }
+  WWB_PD void store(const Grp&, const SrceGroup<0, false>& x, const SlotList&) { x.sh[0].state = kIdle; }
 };
 
 /// W3SRCE for one point by one thread (the host build).
 inline void srce_point(const Cta&, const SrceCtx& x) {
   const Grp c{0, 1};
-  const SrceGroup<0> g{x.p, x.g, x.q, x.f, x.n, x.L, x.w, x.gw, x.w + x.L->common + x.L->ws, x.sh, 1, nullptr};
+  const SrceGroup<0, false> g{x.p, x.g, x.q, x.f, x.n, x.L, x.w, x.gw, x.w + x.L->common + x.L->ws, x.sh, 1, nullptr};
   OnePoint src{x.in};
   srce_run(c, g, src);
 }

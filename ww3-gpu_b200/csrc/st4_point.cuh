@@ -108,6 +108,7 @@ struct Fields {
   /// CUMULW as a function of (IK2, IK, J - ITH), where the registered table is one: CUMULW((IK2-1)
   /// NTH + J, (IK-1) NTH + ITH) = cumt[((IK2-1) NK + IK-1) (2 NTH - 1) + J - ITH + NTH - 1]; else null.
   const float* cumt;
+  int trig_rows;   ///< ECOS and ESIN repeat their first NTH values over NSPEC
   int cum_finite;  ///< every CUMULW value is finite
   int nsat_eff;  ///< SATWEIGHTS rows up to the last that is not zero for the same bin as those after it
   const float *dcki, *qbi;  ///< (NKHS, NKD)

@@ -174,6 +174,16 @@ inline std::vector<float> toeplitz_cumulw(const GridReg& g) {
   return t;
 }
 
+inline bool repeated_trig(const GridReg& g) {
+  for (int id : {A_ECOS, A_ESIN}) {
+    const std::vector<float>& v = g.a[id].f;
+    for (int ik = 1; ik < g.p.nk; ++ik)
+      if (std::memcmp(v.data(), v.data() + static_cast<size_t>(ik) * g.p.nth, sizeof(float) * g.p.nth))
+        return false;
+  }
+  return true;
+}
+
 inline bool finite_cumulw(const GridReg& g) {
   for (float v : g.a[A_CUMULW].f)
     if (!std::isfinite(v)) return false;
@@ -203,6 +213,7 @@ struct FieldPtrs {
       *qbi, *taut, *tauhft, *tauhft2, *fwtable;
   const int *sati_t, *iktab;
   const float* cumt = nullptr;
+  bool trig_rows = false;   ///< ECOS and ESIN repeat their first NTH values (pt::Fields::trig_rows)
   bool cum_finite = false;  ///< every value of the registered CUMULW is finite
   int nsat_eff = -1;  ///< sat_rows of the registration the pointers belong to (-1: every row)
 };
@@ -224,6 +235,7 @@ inline pt::Fields make_fields(const GridReg& g, const FieldPtrs& q) {
   f.cumulw = q.cumulw_t;
   f.cumulw_ld = g.a[A_CUMULW].ext[0];
   f.cumt = q.cumt;
+  f.trig_rows = q.trig_rows ? 1 : 0;
   f.cum_finite = q.cum_finite ? 1 : 0;
   f.nsat_eff = q.nsat_eff < 0 ? f.nsat : q.nsat_eff;
   f.dcki = q.dcki;

@@ -178,12 +178,11 @@ template <class G>
 __device__ __forceinline__ void tail_warp(const G& x, pt::TailBox& box) {
   const int lane = threadIdx.x & 31;
   for (;;) {
-    asm volatile("bar.sync %0, %1;" ::"n"(pt::kBarTail), "n"(kSrceBlock) : "memory");
+    pt::barrier_sync<pt::kBarTail>(kSrceBlock);
     if (box.exit) break;
     const pt::SlotList l = box.l;
     pt::sin4_close(lane, x, l, [] { __syncwarp(); });
-    __threadfence_block();
-    asm volatile("bar.arrive %0, %1;" ::"n"(pt::kBarTailDone), "n"(kSrceBlock) : "memory");
+    pt::barrier_arrive<pt::kBarTailDone>(kSrceBlock);
   }
 }
 __device__ __forceinline__ void tail_exit(const pt::Grp& c, pt::TailBox& box) {
@@ -194,7 +193,7 @@ __device__ __forceinline__ void tail_exit(const pt::Grp& c, pt::TailBox& box) {
 
 /// W3SRCE over the points of one grid. The grid's parameters and table pointers are a kernel parameter,
 /// so the phases read them from the constant bank instead of loading them for every bin.
-template <int NTH>
+template <int NTH, bool PLAIN>
 __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
     const __grid_constant__ SrceDev dev, const __grid_constant__ SrceJob job, int ns, int* counter,
     float* scratch) {
@@ -212,8 +211,8 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
   }
   __syncthreads();
   float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
-  const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
-                             w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns, &box};
+  const pt::SrceGroup<NTH, PLAIN> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
+                                    w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns, &box};
   if (threadIdx.x >= kSrceBlock - 32) {
     tail_warp(x, box);
     return;
@@ -244,7 +243,7 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
   __syncthreads();
   if (threadIdx.x >= kSrceBlock - 32) {
     // The grid's parameters change only between jobs, when no tail is under way.
-    const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L, w, nullptr,
+    const pt::SrceGroup<NTH, false> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L, w, nullptr,
                                nullptr, sh, ns, &box};
     tail_warp(x, box);
     return;
@@ -276,7 +275,7 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
     }
     c.sync();
     float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
-    const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
+    const pt::SrceGroup<NTH, false> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
                                w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns, &box};
     QueuePoints src{ctl, total, counter};
     pt::srce_run(c, x, src);
@@ -287,8 +286,12 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
 using OneKernel = void (*)(SrceDev, SrceJob, int, int*, float*);
 using MultiKernel = void (*)(const SrceJob*, int, int, int, int*, float*);
 /// The kernels built for a number of directions: WW3's usual 36 and 24, else the general ones.
+template <bool PLAIN>
 OneKernel one_kernel(int nth) {
-  return nth == 36 ? srce_kernel<36> : nth == 24 ? srce_kernel<24> : srce_kernel<0>;
+  return nth == 36 ? srce_kernel<36, PLAIN> : nth == 24 ? srce_kernel<24, PLAIN> : srce_kernel<0, PLAIN>;
+}
+OneKernel one_kernel(const pt::SrceLayout& L) {
+  return L.plain ? one_kernel<true>(L.nth) : one_kernel<false>(L.nth);
 }
 MultiKernel multi_kernel(int nth) {
   return nth == 36 ? srce_multi_kernel<36> : srce_multi_kernel<0>;
@@ -324,7 +327,7 @@ struct SrcePlan {
 int srce_per_sm(const pt::SrceLayout& L, int ns, bool multi = false) {
   const size_t smem = srce_smem(L, ns);
   const void* const k = multi ? reinterpret_cast<const void*>(multi_kernel(L.nth))
-                              : reinterpret_cast<const void*>(one_kernel(L.nth));
+                              : reinterpret_cast<const void*>(one_kernel(L));
   WWB_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
   int per_sm = 0;
@@ -364,10 +367,10 @@ void srce_reserve_plan(const pt::SrceLayout& L, const SrcePlan& plan, SrceWork& 
     work.scratch_n = need;
   }
 }
-void set_carveout(int nth, int pct) {
-  WWB_CHECK(cudaFuncSetAttribute(reinterpret_cast<const void*>(one_kernel(nth)),
+void set_carveout(const pt::SrceLayout& L, int pct) {
+  WWB_CHECK(cudaFuncSetAttribute(reinterpret_cast<const void*>(one_kernel(L)),
                                  cudaFuncAttributePreferredSharedMemoryCarveout, pct));
-  WWB_CHECK(cudaFuncSetAttribute(reinterpret_cast<const void*>(multi_kernel(nth)),
+  WWB_CHECK(cudaFuncSetAttribute(reinterpret_cast<const void*>(multi_kernel(L.nth)),
                                  cudaFuncAttributePreferredSharedMemoryCarveout, pct));
 }
 bool srce_reserved(const pt::SrceLayout& L, const SrcePlan& plan, const SrceWork& work) {
@@ -382,7 +385,7 @@ int srce_max_ctas_per_sm(const pt::SrceLayout& L) {
     throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
   const int keep = g_srce_ctas_per_sm;
   g_srce_ctas_per_sm = 0;
-  set_carveout(L.nth, cudaSharedmemCarveoutDefault);
+  set_carveout(L, cudaSharedmemCarveoutDefault);
   const int all = srce_per_sm(L, srce_max_slots(L));
   srce_set_ctas_per_sm(L, keep);  // the carveout of the current choice again
   return all;
@@ -400,7 +403,7 @@ void srce_set_ctas_per_sm(const pt::SrceLayout& L, int ctas) {
     pct = static_cast<int>((100 * ctas * per_cta + 228 * 1024 - 1) / (228 * 1024));
     if (pct > 100) pct = 100;
   }
-  set_carveout(L.nth, pct);
+  set_carveout(L, pct);
 }
 
 size_t srce_smem_bytes(const pt::SrceLayout& L) {
@@ -484,7 +487,7 @@ void launch_srce(const SrceDev& dev, SrceStep step, int npts, float* spec, const
   WWB_CHECK(cudaMemsetAsync(work.counter, 0, sizeof(int), st));
   const SrceJob job{nullptr, step, npts,     0,      spec,   jsea, wn1, cg1,
                     pin,     psc,  whitecap, taubbl, tauice, shave};
-  one_kernel(L.nth)<<<plan.grid, kSrceBlock, plan.smem, st>>>(dev, job, plan.ns, work.counter,
+  one_kernel(L)<<<plan.grid, kSrceBlock, plan.smem, st>>>(dev, job, plan.ns, work.counter,
                                                               work.scratch);
   WWB_CHECK(cudaGetLastError());
 }
