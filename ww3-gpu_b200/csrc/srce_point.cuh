@@ -54,7 +54,7 @@ struct SrceIn {
 };
 
 /// Points a CTA integrates side by side.
-constexpr int kSlots = 4;
+constexpr int kSlots = 8;
 
 enum SlotState : int { kIdle = 0, kFresh1 = 1, kFresh2 = 2, kRun = 3, kDone = 4 };
 
@@ -248,7 +248,14 @@ struct SlotList {
     ++n;
   }
   WWB_PD int at(int j) const { return (ids >> (4 * j)) & 15; }
+  /// Entries j .. j + most - 1 of the list.
+  WWB_PD SlotList part(int j, int most) const {
+    return SlotList{n - j < most ? n - j : most, ids >> (4 * j)};
+  }
 };
+static_assert(kSlots <= 8, "SlotList holds eight 4-bit numbers");
+/// Slots that W3SDS4's sums over tables take together, so that a table row is read once for all of them.
+constexpr int kTogether = 4;
 
 /// What the working warps leave for the tail warp.
 struct TailBox {
@@ -368,30 +375,21 @@ WWB_UNROLL(1)
     }
   }
 }
-/// f(slot, i) for every bin i < n of the listed slots: a warp takes kLanes consecutive bins of
-/// one slot, so what depends on the slot only is uniform in the warp.
+/// f(slot, i) for every bin i < n of the listed slots.
 template <class F>
 WWB_PD void each_bin(const Grp& c, const SlotList& l, int n, F f) {
-  const int nch = (n + Grp::kLanes - 1) / Grp::kLanes, all = l.n * nch;
-WWB_UNROLL(1)
-  for (int e = c.warp(); e < all; e += c.nwarp()) {
-    const int j = (e >= nch) + (e >= 2 * nch) + (e >= 3 * nch);
-    const int i = (e - j * nch) * Grp::kLanes + c.lane();
-    one_copy();
-    if (i < n) f(l.at(j), i);
-  }
+  bins(c, l, n, [](int k) { return k; }, [&](int k, int i) { f(k, i); });
 }
 /// f(slot, r) for r < n of the listed slots, one pair per thread.
 template <class F>
 WWB_PD void each_row(const Grp& c, const SlotList& l, int n, F f) {
 WWB_UNROLL(1)
   for (int e = c.tid; e < l.n * n; e += c.nthr) {
-    const int j = (e >= n) + (e >= 2 * n) + (e >= 3 * n);
+    const int j = e / n;
     one_copy();
     f(l.at(j), e - j * n);
   }
 }
-static_assert(kSlots <= 4, "each_bin and each_row count three slot boundaries");
 /// f(slot) on warp r: lane k runs the k-th listed slot's chain.
 template <class F>
 WWB_PD void each_chain(const Grp& c, int r, const SlotList& l, F f) {
@@ -1172,7 +1170,7 @@ WWB_UNROLL(1)
       const float dely = x.w[L.tail + 7 * kJtot];
 WWB_UNROLL(1)
       for (int e = lane; e < l.n * kJtot; e += Grp::kLanes) {
-        const int n = (e >= kJtot) + (e >= 2 * kJtot) + (e >= 3 * kJtot), k = l.at(n), j = e - n * kJtot;
+        const int n = e / kJtot, k = l.at(n), j = e - n * kJtot;
         float* const t = x.s(k, L.jt);
         const float w = (j == 0 || j == kJtot - 1) ? 0.5f : 1.0f;
         const float lev = p.sintailpar[2] > 0.0f ? t[kLev + j] : x.sh[k].levtail0;
@@ -1766,9 +1764,13 @@ WWB_PD void srce_sds4(const Grp& c, const G& x, const SlotList& l) {
       // Rows of SATWEIGHTS past nsat_eff are all zero for one and the same bin: adding 0 * A once has
       // the effect of adding it for each of them.
       const int rows = f.nsat_eff < f.nsat ? f.nsat_eff + 1 : f.nsat;
-      if (l.n == 1) sat_sums<1>(c, x, l, rows, ik1);
-      else if (l.n == 2) sat_sums<2>(c, x, l, rows, ik1);
-      else sat_sums<kSlots>(c, x, l, rows, ik1);
+WWB_UNROLL(1)
+      for (int j = 0; j < l.n; j += kTogether) {
+        one_copy();
+        const SlotList g = l.part(j, kTogether);
+        if (g.n == 1) sat_sums<1>(c, x, g, rows, ik1);
+        else sat_sums<kTogether>(c, x, g, rows, ik1);
+      }
       c.sync();
     }
     each_row(c, l, nk, [&](int k, int ik0) {
@@ -2153,9 +2155,13 @@ WWB_UNROLL(1)
     c.sync();
   }
   if (turb) {
-    if (l.n == 1) sds4_turb<1>(c, x, l, blocks, dikcumul, ik1, R + kA1 * K, R + kRen * K);
-    else if (l.n == 2) sds4_turb<2>(c, x, l, blocks, dikcumul, ik1, R + kA1 * K, R + kRen * K);
-    else sds4_turb<kSlots>(c, x, l, blocks, dikcumul, ik1, R + kA1 * K, R + kRen * K);
+WWB_UNROLL(1)
+    for (int j = 0; j < l.n; j += kTogether) {
+      one_copy();
+      const SlotList g = l.part(j, kTogether);
+      if (g.n == 1) sds4_turb<1>(c, x, g, blocks, dikcumul, ik1, R + kA1 * K, R + kRen * K);
+      else sds4_turb<kTogether>(c, x, g, blocks, dikcumul, ik1, R + kA1 * K, R + kRen * K);
+    }
   }
   c.sync();
   if (wcap) {

@@ -39,8 +39,8 @@ constexpr int kSt4Block = 256;
 
 /// Threads of a W3SRCE CTA (the last warp forms the tails), and the CTAs per SM it is built for: one
 /// CTA's ordered chains run beside the other's parallel phases.
-constexpr int kSrceBlock = 384;
-constexpr int kSrceMinBlocks = 2;
+constexpr int kSrceBlock = 768;
+constexpr int kSrceMinBlocks = 1;
 
 /// One grid's W3SRCE work buffers: the work queue's counter and the global part of the resident
 /// CTAs' working sets (grow-only; it stays in L2 at these sizes). Owned by the grid's context.
