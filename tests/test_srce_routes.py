@@ -1,0 +1,114 @@
+"""The routes W3SRCE's kernel takes by a rule, against the general ones: on the CPU the tables derived
+from the registered ones and the branch-free libm forms (bit for bit), on the GPU the kernel's forms (36,
+24 and other numbers of directions, with and without sheltering, numbers of points around the slots
+and CTAs) against the host build of the same source, one point at a time."""
+
+import ctypes
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import cuda_available
+import st4_common as sc
+
+P = ctypes.c_void_p
+
+
+@pytest.fixture(scope="module")
+def routes(tmp_path_factory):
+    so = tmp_path_factory.mktemp("routes") / "libroutes.so"
+    csrc = sc.ROOT / "ww3-gpu_b200" / "csrc"
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O2", "-march=x86-64-v3", "-ffp-contract=off",
+                    "-fno-math-errno", "-fPIC", "-shared", f"-I{csrc}", "-I/usr/local/cuda/include",
+                    str(sc.ROOT / "tests" / "srce_routes.cpp"), str(csrc / "snl1_tables.cpp"), "-o",
+                    str(so)], check=True)
+    H = ctypes.CDLL(str(so))
+    H.hemu_st4_init.argtypes = [P, sc.I, P, sc.I]
+    for f in (H.hemu_st4_set_real, H.hemu_st4_set_int):
+        f.argtypes = [sc.I, P, sc.I, P, P]
+    H.hemu_snl1_init.argtypes = [sc.I, sc.I] + [sc.F] * 10 + [P]
+    H.hemu_srce_init.argtypes = [P, sc.I, P, sc.I, P, P, P, P, P]
+    H.hemu_srce_batch.argtypes = [sc.I] * 4 + [sc.F, sc.I] + [P] * 9
+    H.routes_libm.argtypes = [ctypes.c_long, ctypes.c_ulonglong, P]
+    return H
+
+
+def config(synth, nk, nth, shelter, ln1=0, seed=0):
+    st = synth.st4_setup(nk, nth, variant="analytic")
+    st["rpar"][st["R"]["TTAUWSHELTER"]] = shelter
+    t = synth.st4_tables_own(st)
+    return st, t, synth.srce_setup(st, ln1=ln1, seed=seed), synth.dia_config(nk, nth)
+
+
+def host_setup(H, synth, st, t, sr, dia, regs=None):
+    assert H.hemu_st4_init(sc.p(st["rpar"]), st["rpar"].size, sc.p(st["ipar"]), st["ipar"].size) == 0
+    for aid, arr, is_int, lb, ext in regs or synth.st4_registrations(st, t):
+        arr = np.ascontiguousarray(arr, np.int32 if is_int else np.float32)
+        lb, ext = np.asarray(lb, np.int32), np.asarray(ext, np.int32)
+        f = H.hemu_st4_set_int if is_int else H.hemu_st4_set_real
+        assert f(aid, sc.p(arr), len(ext), sc.p(lb), sc.p(ext)) == 0
+    assert H.hemu_st4_commit() == 0
+    cfg, sig = dia
+    assert H.hemu_snl1_init(cfg["nk"], cfg["nth"], *[cfg[k] for k in sc.NK_ARGS], sc.p(sig)) == 0
+    assert H.hemu_srce_init(sc.p(sr["rpar"]), len(sr["rpar"]), sc.p(sr["ipar"]), len(sr["ipar"]),
+                            *[sc.p(sr[k]) for k in ("sig", "dden", "ecos", "esin", "mapwn")]) == 0
+
+
+def same(a, b):
+    return {k: int((np.ascontiguousarray(a[k]).view(np.uint32) != np.ascontiguousarray(b[k]).view(np.uint32)).sum())
+            for k in a}
+
+
+@pytest.mark.parametrize("nk,nth", [(25, 24), (13, 7), (12, 10)])
+def test_derived_tables_change_no_bit(routes, synth, nk, nth):
+    st, t, sr, dia = config(synth, nk, nth, 0.0)
+    host_setup(routes, synth, st, t, sr, dia)
+    pts = synth.srce_points(5, seed=nk, nk=nk, nth=nth, depth_range=(2.0, 4000.0))
+    pts["pin"][0, 2] = 0.0  # a wind along an axis leaves the stress scan's parallel form
+    be = sc.hemu_backend(routes)
+    assert routes.routes_derived(0) & 7 == 7
+    general = be.srce_batch(pts)
+    routes.routes_derived(1)
+    assert not any(same(general, be.srce_batch(pts)).values())
+
+
+def test_derived_tables_are_refused_where_they_do_not_apply(routes, synth):
+    st, t, sr, dia = config(synth, 12, 10, 0.0)
+    for key, at, value, bit in (("cumulw", 7 * 120 + 13, 0.5, 1), ("cumulw", 3, np.inf, 2)):
+        t2 = dict(t, cumulw=t["cumulw"].copy())
+        t2[key][at] = value
+        host_setup(routes, synth, st, t2, sr, dia)
+        assert routes.routes_derived(1) & bit == 0
+    regs = [list(r) for r in synth.st4_registrations(st, t)]
+    regs[6][1] = np.array(regs[6][1], copy=True)
+    regs[6][1][25] += np.float32(1e-3)  # ECOS of another row
+    host_setup(routes, synth, st, t, sr, dia, regs)
+    assert routes.routes_derived(1) & 4 == 0
+
+
+def test_branch_free_libm_equals_general(routes):
+    bad = np.zeros(7, np.int64)
+    routes.routes_libm(3_000_000, 88172645463325252, sc.p(bad))
+    assert not bad.any(), bad
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+@pytest.mark.parametrize("nk,nth,shelter,ln1,seed,sizes", [
+    (36, 36, 0.0, 0, 0, (1, 9)), (25, 24, 0.0, 1, 1, (1, 8, 150)), (25, 24, 0.3, 0, 0, (7, 300)),
+    (36, 36, 0.3, 0, 1, (3,)), (13, 7, 0.0, 0, 0, (1, 1185)), (12, 10, 0.3, 1, 0, (17, 1300))])
+def test_kernel_forms_equal_host_build(pkg, routes, synth, nk, nth, shelter, ln1, seed, sizes):
+    st, t, sr, dia = config(synth, nk, nth, shelter, ln1, seed)
+    host_setup(routes, synth, st, t, sr, dia)
+    routes.routes_derived(0)
+    host = sc.hemu_backend(routes)
+    grid = pkg.SrceGrid(950 + nk, st["rpar"], st["ipar"], synth.st4_registrations(st, t), *dia, sr)
+    gpu = sc.Backend(lambda name: (lambda *a: getattr(grid.L, "ww_" + name)(grid.igrid, *a)))
+    for n in sizes:
+        pts = synth.srce_points(n, seed=n, nk=nk, nth=nth, depth_range=(5.0, 4000.0))
+        pts["pin"][0, 2] = 0.0
+        # Fewer substeps a point keep the host build's share short.
+        r, g = host.srce_batch(pts, dtg=60.0), gpu.srce_batch(pts, dtg=60.0)
+        assert grid.L.ww_srce_last_error() == 0
+        assert not any(same(r, g).values()), (n, same(r, g))

@@ -12,6 +12,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -159,15 +160,18 @@ inline std::vector<float> toeplitz_cumulw(const GridReg& g) {
   const int nk = g.p.nk, nth = g.p.nth, ld = 2 * nth - 1;
   const size_t n = c.ext[0];
   std::vector<float> t(static_cast<size_t>(nk) * nk * ld, 0.0f);
+  // Column by column, as the table lies in memory.
   for (int ik = 0; ik < nk; ++ik)
-    for (int ik2 = 0; ik2 < nk; ++ik2) {
-      float* const row = t.data() + (static_cast<size_t>(ik2) * nk + ik) * ld + nth - 1;
-      for (int ith = 0; ith < nth; ++ith) {
-        const float* const col =
-            c.f.data() + static_cast<size_t>(ik2) * nth + (static_cast<size_t>(ik) * nth + ith) * n;
-        for (int j = 0; j < nth; ++j) {
-          if (ith == 0 || j == 0) row[j - ith] = col[j];  // the first value of each J - ITH
-          else if (std::memcmp(&row[j - ith], &col[j], sizeof(float)) != 0) return {};
+    for (int ith = 0; ith < nth; ++ith) {
+      const float* const col = c.f.data() + (static_cast<size_t>(ik) * nth + ith) * n;
+      for (int ik2 = 0; ik2 < nk; ++ik2) {
+        float* const row = t.data() + (static_cast<size_t>(ik2) * nk + ik) * ld + nth - 1 - ith;
+        const float* const from = col + static_cast<size_t>(ik2) * nth;
+        if (ith == 0) {
+          std::memcpy(row, from, sizeof(float) * nth);
+        } else {
+          row[0] = from[0];  // the first value of J - ITH = -ITH; the others were met before
+          if (std::memcmp(row + 1, from + 1, sizeof(float) * (nth - 1)) != 0) return {};
         }
       }
     }
@@ -185,9 +189,9 @@ inline bool repeated_trig(const GridReg& g) {
 }
 
 inline bool finite_cumulw(const GridReg& g) {
-  for (float v : g.a[A_CUMULW].f)
-    if (!std::isfinite(v)) return false;
-  return true;
+  int bad = 0;
+  for (float v : g.a[A_CUMULW].f) bad |= !(std::fabs(v) <= std::numeric_limits<float>::max());
+  return bad == 0;
 }
 
 /// SATWEIGHTS rows to sum: from the returned row on, every row is zero with the same SATINDICES as
