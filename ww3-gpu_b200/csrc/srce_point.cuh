@@ -14,7 +14,9 @@
 // can do and some fifteen ordered chains (sums over 1296 bins, Newton steps, the stress scan
 // over frequency, the 50-step tail) that one thread does. With one point per CTA the chains leave
 // 127 of 128 threads at a barrier and the four CTAs of an SM evict each other's code from the
-// instruction cache: 36 x 36 bins, 9,520 points took 419 ms, 27.7 ms for a launch of 5 points.
+// instruction cache: on B200, 36 x 36 bins, 9,520 points took 422 ms and a launch of 5 points 24.8 ms;
+// in slots 99 ms and 4.4 ms. What bounds it now: instruction issue (about 2 of 4 per cycle) and fetch (two
+// CTAs of 384 threads and four slots per SM, in two phases at a time: 106 ms; three: 158 ms).
 // Here a CTA holds up to kSlots points in slots. A phase is either a loop over all (slot, bin) or
 // (slot, frequency) pairs by all warps, or a set of roles: role r is warp r, its lane k the chain of
 // slot k, so the chains of all slots and roles run at the same time and one instruction serves
@@ -53,7 +55,9 @@ struct SrceIn {
   float d_inp, u10abs, u10dir, as, ice, dtg, dair, coef;
 };
 
-/// Points a CTA integrates side by side.
+/// Points a CTA integrates side by side: a chain phase costs the same for eight as for one, and their
+/// working sets (22 KB each at 36 x 36) fill the SM's shared memory. One CTA of four per SM ran 167 ms for
+/// 9,520 points where two of four ran 133; one of eight ran 98.7 where two of four ran 106.
 constexpr int kSlots = 8;
 
 enum SlotState : int { kIdle = 0, kFresh1 = 1, kFresh2 = 2, kRun = 3, kDone = 4 };
@@ -254,7 +258,8 @@ struct SlotList {
   }
 };
 static_assert(kSlots <= 8, "SlotList holds eight 4-bit numbers");
-/// Slots that W3SDS4's sums over tables take together, so that a table row is read once for all of them.
+/// Slots that W3SDS4's sums over tables take together, so that a table row is read once for all of them
+/// (9,520 points: two 101 ms, four 98.7, eight 98; 777 points with Romero's breaking: 18.2, 18.5, 19.1).
 constexpr int kTogether = 4;
 
 /// What the working warps leave for the tail warp.
@@ -879,7 +884,7 @@ WWB_PD ScanK scan_k(const G& x, const Sin4At& at, const float* tr, int ik, float
 }
 
 /// Lanes that share one point's stress scan: 36 directions in three rounds, 24 in two; two points
-/// to a warp.
+/// to a warp (18 lanes and one point: no faster at 36 directions, 6 % slower at 24).
 #if defined(__CUDA_ARCH__)
 constexpr int kScanLanes = 12;
 #else
