@@ -4,6 +4,7 @@ from the registered ones and the branch-free libm forms (bit for bit), on the GP
 and CTAs) against the host build of the same source, one point at a time."""
 
 import ctypes
+import re
 import subprocess
 
 import numpy as np
@@ -91,6 +92,15 @@ def test_branch_free_libm_equals_general(routes):
     bad = np.zeros(7, np.int64)
     routes.routes_libm(3_000_000, 88172645463325252, sc.p(bad))
     assert not bad.any(), bad
+
+
+def test_named_barriers_do_not_ask_for_a_converged_warp():
+    """bar.sync and bar.arrive are the .aligned forms: all lanes have to issue them together, which the
+    W3SRCE kernels' code before them does not guarantee."""
+    csrc = sc.ROOT / "ww3-gpu_b200" / "csrc"
+    text = "".join((csrc / f).read_text() for f in ("srce_point.cuh", "st4_srce_kernel.cu"))
+    named = re.findall(r'asm volatile\("(bar[a-z.]*) ', text)
+    assert sorted(named) == ["barrier.arrive", "barrier.sync"]
 
 
 @pytest.mark.gpu

@@ -179,20 +179,23 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
 }
 
 /// The named barriers of a CTA: its working warps' own, and the two over which they hand the tail to the
-/// tail warp and take its results. bar.sync and bar.arrive want the warp's lanes together, and nothing
-/// makes the compiler rejoin them before inline assembly, so __syncwarp comes directly before.
+/// tail warp and take its results. They follow code in which lanes diverge, and nothing makes a warp's
+/// lanes issue an inline assembly statement together (__syncwarp only makes them meet before it), so
+/// these are PTX's barrier.sync and barrier.arrive, which do not ask for that; bar.sync and bar.arrive
+/// are their .aligned forms, which do, and a warp that came apart could pass early or wait for good.
+/// __syncwarp keeps the usual case one instruction for the warp.
 constexpr int kBarWork = 1, kBarTail = 2, kBarTailDone = 3;
 #if defined(__CUDACC__)
 template <int ID>
 __device__ __forceinline__ void barrier_sync(int threads) {
   __syncwarp();
-  asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(threads) : "memory");
+  asm volatile("barrier.sync %0, %1;" ::"n"(ID), "r"(threads) : "memory");
 }
 template <int ID>
 __device__ __forceinline__ void barrier_arrive(int threads) {
   __threadfence_block();
   __syncwarp();
-  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "r"(threads) : "memory");
+  asm volatile("barrier.arrive %0, %1;" ::"n"(ID), "r"(threads) : "memory");
 }
 #endif
 
