@@ -15,8 +15,9 @@
 // over frequency, the 50-step tail) that one thread does. With one point per CTA the chains leave
 // 127 of 128 threads at a barrier and the four CTAs of an SM evict each other's code from the
 // instruction cache: on B200, 36 x 36 bins, 9,520 points took 422 ms and a launch of 5 points 24.8 ms;
-// in slots 99 ms and 4.4 ms. What bounds it now: instruction issue (about 2 of 4 per cycle) and fetch (two
-// CTAs of 384 threads and four slots per SM, in two phases at a time: 106 ms; three: 158 ms).
+// in slots 102 ms and 4.5 ms. What bounds it now: instruction issue (about 2 of 4 per cycle) and fetch (two
+// CTAs of four slots per SM, in two phases at a time, ran 7 % longer than one of eight, three of three
+// slots 60 % longer; both measured with fewer registers per thread than now).
 // Here a CTA holds up to kSlots points in slots. A phase is either a loop over all (slot, bin) or
 // (slot, frequency) pairs by all warps, or a set of roles: role r is warp r, its lane k the chain of
 // slot k, so the chains of all slots and roles run at the same time and one instruction serves
@@ -57,7 +58,8 @@ struct SrceIn {
 
 /// Points a CTA integrates side by side: a chain phase costs the same for eight as for one, and their
 /// working sets (22 KB each at 36 x 36) fill the SM's shared memory. One CTA of four per SM ran 167 ms for
-/// 9,520 points where two of four ran 133; one of eight ran 98.7 where two of four ran 106.
+/// 9,520 points where two of four ran 133; one of eight ran 98.7 where two of four ran 106 (taken on the
+/// way here, with 768 threads; now 102).
 constexpr int kSlots = 8;
 
 enum SlotState : int { kIdle = 0, kFresh1 = 1, kFresh2 = 2, kRun = 3, kDone = 4 };

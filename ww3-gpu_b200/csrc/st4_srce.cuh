@@ -38,9 +38,10 @@ struct SrceStep {
 constexpr int kSt4Block = 256;
 
 /// Threads of a W3SRCE CTA (the last warp forms the tails), and the CTAs per SM it is built for: one,
-/// so that every warp of an SM runs the same phase's code (9,520 points: 98.7 ms; 640 threads 99.8, 1,024
-/// threads 100.5; two CTAs of 384 with four slots 106, three of 256 with three 158).
-constexpr int kSrceBlock = 768;
+/// so that every warp of an SM runs the same phase's code. 512 threads leave 128 registers each, so
+/// little is spilled across the barriers: 9,520 points 101-102 ms; 384 threads 106, 448 107, 480 105.5,
+/// 544 106, 640 108, 768 107.5, 1,024 108; a launch of 5 points 4.5 ms against 4.8 with 768.
+constexpr int kSrceBlock = 512;
 constexpr int kSrceMinBlocks = 1;
 
 /// One grid's W3SRCE work buffers: the work queue's counter and the global part of the resident
