@@ -4,6 +4,7 @@
 // the general ones. Compiled by tests/test_srce_routes.py.
 #include "hemu.cpp"
 
+#include <algorithm>
 #include <cstdint>
 
 extern "C" {
@@ -19,6 +20,13 @@ int routes_derived(int on) {
   g_fields.trig_rows = on && trig;
   g_fields.nsat_eff = on ? rows : g_fields.nsat;
   return (cumt.empty() ? 0 : 1) | (fin ? 2 : 0) | (trig ? 4 : 0) | (rows < g_fields.nsat ? 8 : 0);
+}
+
+/// The bytes of the working set's layout (at most cap of them); returns their number.
+int routes_layout(unsigned char* out, int cap) {
+  const pt::SrceLayout L = pt::srce_layout(g_p, g_ndev);
+  std::memcpy(out, &L, std::min<size_t>(cap, sizeof L));
+  return static_cast<int>(sizeof L);
 }
 
 /// Mismatches over n seeded arguments of: 0 div_core (reciprocal seed an ulp off either way), 1 expf_q /

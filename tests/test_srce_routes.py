@@ -94,6 +94,19 @@ def test_branch_free_libm_equals_general(routes):
     assert not bad.any(), bad
 
 
+def test_working_set_layout_depends_on_the_spectral_grid_only(routes, synth):
+    """ww_steps_fuse takes grids whose layouts are equal: ST4's options must not show in them."""
+    seen = set()
+    for shelter, case, stab3 in ((0.0, 1.0, 0), (0.3, 1.0, 0), (0.0, 3.0, 0), (0.0, 1.0, 1)):
+        st, t, sr, dia = config(synth, 12, 10, shelter)
+        st["rpar"][st["R"]["SSDSC"]] = case
+        st["ipar"][6] = stab3
+        host_setup(routes, synth, st, t, sr, dia)
+        buf = np.zeros(4096, np.uint8)
+        seen.add(bytes(buf[:routes.routes_layout(sc.p(buf), buf.size)]))
+    assert len(seen) == 1
+
+
 def test_named_barriers_do_not_ask_for_a_converged_warp():
     """bar.sync and bar.arrive are the .aligned forms: all lanes have to issue them together, which the
     W3SRCE kernels' code before them does not guarantee."""
@@ -101,6 +114,52 @@ def test_named_barriers_do_not_ask_for_a_converged_warp():
     text = "".join((csrc / f).read_text() for f in ("srce_point.cuh", "st4_srce_kernel.cu"))
     named = re.findall(r'asm volatile\("(bar[a-z.]*) ', text)
     assert sorted(named) == ["barrier.arrive", "barrier.sync"]
+
+
+needs_gpu = pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+
+
+@pytest.mark.gpu
+@needs_gpu
+def test_grids_of_different_st4_options_fuse(pkg, synth):
+    """One launch over the points of three grids of one spectral size whose ST4 parameters differ gives
+    every grid the spectra of its own recorded step."""
+    def record(base):
+        grids, vas, steps = [], [], []
+        for j, (shelter, n) in enumerate(((0.0, 1300), (0.3, 40), (0.0, 9))):
+            st, t, sr, dia = config(synth, 25, 24, shelter)
+            if j == 2:
+                st["rpar"][st["R"]["SSDSC"] + 2] = 0.4  # the isotropic cumulative term
+            g = pkg.SrceGrid(base + j, st["rpar"], st["ipar"], synth.st4_registrations(st, t), *dia, sr)
+            p = synth.srce_points(n, seed=7 * j, nk=25, nth=24, depth_range=(5.0, 4000.0))
+            va = np.zeros((n + 1, 600), np.float32)
+            va[1:] = p["spec"]
+            jsea = np.arange(n, 0, -1, dtype=np.int32)
+            with pkg.Step(base + j) as step:
+                g.batch_va(n, va, jsea, *[p[k] for k in ("wn1", "cg1", "pin", "psc", "whitecap", "taubbl",
+                                                         "tauice")], np.zeros(n, np.int32), dtg=300.0)
+            grids.append(g), vas.append(va), steps.append(step)
+        return vas, steps
+
+    def read(base, vas):
+        for j, va in enumerate(vas):
+            assert pkg.va_host_read(base + j, va) == 0
+
+    own, steps = record(970)
+    for s in steps:
+        s.run(2)
+    read(970, own)
+    before, fsteps = record(980)
+    start = [va.copy() for va in before]
+    pkg.steps_fuse([980, 981, 982])
+    pkg.steps_run([980, 981, 982], 2)
+    pkg.steps_fuse([])
+    read(980, before)
+    for j in range(3):
+        assert np.array_equal(own[j].view(np.uint32), before[j].view(np.uint32)), j
+        assert not np.array_equal(start[j], before[j])
+    for s in steps + fsteps:
+        s.free()
 
 
 @pytest.mark.gpu

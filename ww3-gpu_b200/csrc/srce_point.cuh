@@ -93,7 +93,6 @@ struct SrceSh {
 /// Offsets (in floats) of the working set; see the file header.
 struct SrceLayout {
   int nspec, nk, nth;
-  int plain;  ///< SSDSC(1) = 1, TTAUWSHELTER = 0 and no W3_STAB3: SrceGroup's PLAIN form
   unsigned nth_magic;  ///< i / nth = umulhi(i, nth_magic) for the bins' range
   // shared: what all slots read, then per slot (stride ws), then the transient region
   int pwsig, pwdir, tail, ec, es, common;
@@ -127,7 +126,6 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
   L.nspec = ns;
   L.nk = nk;
   L.nth = nth;
-  L.plain = nint(q.ssdsc[0]) == 1 && q.ttauwshelter == 0.0f && !q.stab3;
   L.nth_magic = static_cast<unsigned>(0x100000000ULL / static_cast<unsigned>(nth)) + 1u;
   int o = 0;
   L.pwsig = o; o += K;
@@ -275,9 +273,8 @@ struct TailBox {
 
 /// What the CTA's phases read: the tables of one grid and the slots' memory. NTH: the number of
 /// directions where the kernel is built for it (bin addresses and the loops over directions are then
-/// compile-time arithmetic), 0 for any. PLAIN: SSDSC(1) = 1 and no sheltering, so the other breaking
-/// forms and the serial stress scan take no part of the kernel's registers and instruction cache.
-template <int NTH, bool PLAIN>
+/// compile-time arithmetic), 0 for any.
+template <int NTH>
 struct SrceGroup {
   const srce::Params* p;
   const SrceGrid* g;
@@ -292,7 +289,6 @@ struct SrceGroup {
   int ns;
   TailBox* box;  ///< null: the tail runs where it is called
   static constexpr int kNth = NTH;
-  static constexpr bool kPlain = PLAIN;
   WWB_PD int nth() const { return NTH ? NTH : L->nth; }
   WWB_PD float* s(int k, int off) const { return w + off + k * L->ws; }
   WWB_PD float* gs(int k, int off) const { return gw + (off + k * L->total_g); }
@@ -1025,12 +1021,6 @@ WWB_UNROLL(1)
   }
 }
 
-/// scan_serial out of line, for the rare slot that needs it in a kernel without sheltering.
-template <class G>
-WWB_PN void scan_serial_call(Grp c, G x, SlotList l, Sin4At at) {
-  scan_serial(c, x, l, at);
-}
-
 /// a / b for b in [2^-20, 2^20], correctly rounded, from y = 1 / b correctly rounded (0: unknown): two steps q + (a - b q) y with fused
 /// multiply-adds (Markstein 1990, IBM J. Res. Dev. 34: one step from a quotient within an ulp is exact,
 /// the first makes it so), where nothing under- or overflows; else the division itself. The tail divides
@@ -1394,8 +1384,7 @@ WWB_UNROLL(1)
   }
   if (ser.n) {
     c.sync();
-    if (G::kPlain) scan_serial_call(c, x, ser, at);
-    else scan_serial(c, x, ser, at);
+    scan_serial(c, x, ser, at);
     c.sync();
   }
   // 3. TAUWX and TAUWY enter the next step's fluxes and W3SPR4 only: the tail warp forms them beside the
@@ -1767,7 +1756,7 @@ WWB_PD void srce_sds4(const Grp& c, const G& x, const SlotList& l) {
     s.sinus = sn;
     s.cosus = cs;
   });
-  const int sdscase = G::kPlain ? 1 : nint(ssdsc[0]);
+  const int sdscase = nint(ssdsc[0]);
   if (sdscase == 1) {
     // 2.a.1 Saturation (:2262-2290).
     if (p.ssdsdth < 180.0f) {
@@ -2861,20 +2850,20 @@ struct SrceCtx {
 struct OnePoint {
   SrceIn in;
   bool taken = false;
-  WWB_PD void load(const Grp&, const SrceGroup<0, false>& x, SlotList& fresh) {
+  WWB_PD void load(const Grp&, const SrceGroup<0>& x, SlotList& fresh) {
     if (taken) return;
     taken = true;
     x.sh[0].in = in;
     x.sh[0].state = in.it != 0 ? kFresh1 : kFresh2;
     fresh.add(0);
   }
-  WWB_PD void store(const Grp&, const SrceGroup<0, false>& x, const SlotList&) { x.sh[0].state = kIdle; }
+  WWB_PD void store(const Grp&, const SrceGroup<0>& x, const SlotList&) { x.sh[0].state = kIdle; }
 };
 
 /// W3SRCE for one point by one thread (the host build).
 inline void srce_point(const Cta&, const SrceCtx& x) {
   const Grp c{0, 1};
-  const SrceGroup<0, false> g{x.p, x.g, x.q, x.f, x.n, x.L, x.w, x.gw, x.w + x.L->common + x.L->ws, x.sh, 1, nullptr};
+  const SrceGroup<0> g{x.p, x.g, x.q, x.f, x.n, x.L, x.w, x.gw, x.w + x.L->common + x.L->ws, x.sh, 1, nullptr};
   OnePoint src{x.in};
   srce_run(c, g, src);
 }

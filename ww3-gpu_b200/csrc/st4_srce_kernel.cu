@@ -193,7 +193,7 @@ __device__ __forceinline__ void tail_exit(const pt::Grp& c, pt::TailBox& box) {
 
 /// W3SRCE over the points of one grid. The grid's parameters and table pointers are a kernel parameter,
 /// so the phases read them from the constant bank instead of loading them for every bin.
-template <int NTH, bool PLAIN>
+template <int NTH>
 __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
     const __grid_constant__ SrceDev dev, const __grid_constant__ SrceJob job, int ns, int* counter,
     float* scratch) {
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_kernel(
   }
   __syncthreads();
   float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
-  const pt::SrceGroup<NTH, PLAIN> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
+  const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
                                     w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns, &box};
   if (threadIdx.x >= kSrceBlock - 32) {
     tail_warp(x, box);
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
   __syncthreads();
   if (threadIdx.x >= kSrceBlock - 32) {
     // The grid's parameters change only between jobs, when no tail is under way.
-    const pt::SrceGroup<NTH, false> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L, w, nullptr,
+    const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L, w, nullptr,
                                nullptr, sh, ns, &box};
     tail_warp(x, box);
     return;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
     }
     c.sync();
     float* const gw = scratch + static_cast<size_t>(blockIdx.x) * ns * dev.L.total_g;
-    const pt::SrceGroup<NTH, false> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
+    const pt::SrceGroup<NTH> x{&dev.p, &dev.g, &dev.q, &dev.f, &dev.n, &dev.L,
                                w,      gw,     w + dev.L.common + ns * dev.L.ws, sh, ns, &box};
     QueuePoints src{ctl, total, counter};
     pt::srce_run(c, x, src);
@@ -286,14 +286,10 @@ __global__ void __launch_bounds__(kSrceBlock, kSrceMinBlocks) srce_multi_kernel(
 using OneKernel = void (*)(SrceDev, SrceJob, int, int*, float*);
 using MultiKernel = void (*)(const SrceJob*, int, int, int, int*, float*);
 /// The kernels built for a number of directions: WW3's usual 36 and 24 (compile-time bin addresses and
-/// unrolled sums), else the general ones; and, for SSDSC(1) = 1 without sheltering, without the other
-/// breaking forms and the serial scan (9,520 points: 105.9 ms against 106.9 with them).
-template <bool PLAIN>
-OneKernel one_kernel(int nth) {
-  return nth == 36 ? srce_kernel<36, PLAIN> : nth == 24 ? srce_kernel<24, PLAIN> : srce_kernel<0, PLAIN>;
-}
+/// unrolled sums), else the general ones. A form of its own for SSDSC(1) = 1 without sheltering gave
+/// nothing (9,520 points: 101.1-102.5 ms with it, 101.3 without).
 OneKernel one_kernel(const pt::SrceLayout& L) {
-  return L.plain ? one_kernel<true>(L.nth) : one_kernel<false>(L.nth);
+  return L.nth == 36 ? srce_kernel<36> : L.nth == 24 ? srce_kernel<24> : srce_kernel<0>;
 }
 MultiKernel multi_kernel(int nth) {
   return nth == 36 ? srce_multi_kernel<36> : srce_multi_kernel<0>;
