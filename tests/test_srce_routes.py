@@ -163,6 +163,40 @@ def test_grids_of_different_st4_options_fuse(pkg, synth):
 
 
 @pytest.mark.gpu
+@needs_gpu
+def test_launches_of_two_threads_do_not_lower_each_others_limits(pkg, synth, capfd):
+    """Two grids on two threads and streams, one with one slot per CTA and one with eight: neither call may
+    be refused by the shared-memory limit that the other has set."""
+    import threading
+
+    import torch
+
+    jobs = []
+    for j, n in enumerate((3, 1200)):
+        st, t, sr, dia = config(synth, 25, 24, 0.0)
+        g = pkg.SrceGrid(990 + j, st["rpar"], st["ipar"], synth.st4_registrations(st, t), *dia, sr)
+        p = synth.srce_points(n, seed=j, nk=25, nth=24, depth_range=(5.0, 4000.0))
+        dev = [torch.from_numpy(np.ascontiguousarray(p[k])).cuda()
+               for k in ("spec", "wn1", "cg1", "pin", "psc", "whitecap", "taubbl", "tauice")]
+        jobs.append((g, n, dev + [torch.zeros(n, dtype=torch.int32, device="cuda")], torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    capfd.readouterr()
+
+    def call(g, n, dev, stream):
+        for _ in range(300):
+            g.L.ww_srce_batch_device(g.igrid, 1, 0, 1, 1, 10.0, n, *[d.data_ptr() for d in dev],
+                                     ctypes.c_void_p(stream.cuda_stream))
+
+    threads = [threading.Thread(target=call, args=job) for job in jobs]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    assert "code" not in capfd.readouterr().err
+
+
+@pytest.mark.gpu
 @pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
 @pytest.mark.parametrize("nk,nth,shelter,ln1,seed,sizes", [
     (36, 36, 0.0, 0, 0, (1, 9)), (25, 24, 0.0, 1, 1, (1, 8, 150)), (25, 24, 0.3, 0, 0, (7, 300)),

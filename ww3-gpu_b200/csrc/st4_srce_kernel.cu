@@ -316,6 +316,10 @@ size_t srce_smem(const pt::SrceLayout& L, int ns) {
 }
 constexpr size_t kSrceStatic =
     sizeof(pt::SrceSh) * pt::kSlots + sizeof(SrceCtl) + sizeof(SrceDev) + sizeof(pt::TailBox) + 64;
+/// The dynamic shared memory that every call allows a W3SRCE kernel: one value for all, never a launch's
+/// own, so that a launch is not refused because another thread's (of fewer slots or a smaller grid) has
+/// lowered the kernel's limit between its plan and its start.
+constexpr size_t kSrceDynMax = (227 * 1024 - kSrceStatic) & ~static_cast<size_t>(15);
 
 /// A W3SRCE launch: slots per CTA, CTAs, shared memory.
 struct SrcePlan {
@@ -327,7 +331,7 @@ int srce_per_sm(const pt::SrceLayout& L, int ns, bool multi = false) {
   const void* const k = multi ? reinterpret_cast<const void*>(multi_kernel(L.nth))
                               : reinterpret_cast<const void*>(one_kernel(L));
   WWB_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem)));
+                                 static_cast<int>(kSrceDynMax)));
   int per_sm = 0;
   WWB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kSrceBlock, smem));
   if (per_sm < 1) throw CudaError(cudaErrorInvalidConfiguration, "srce occupancy");
@@ -335,9 +339,8 @@ int srce_per_sm(const pt::SrceLayout& L, int ns, bool multi = false) {
 }
 /// Slots a CTA of this layout can have: all of them where as many CTAs fit an SM as with one.
 int srce_max_slots(const pt::SrceLayout& L) {
-  const size_t budget = 233472 / kSrceMinBlocks - 1024;
   for (int ns = pt::kSlots; ns > 1; --ns)
-    if (srce_smem(L, ns) + kSrceStatic <= budget) return ns;
+    if (srce_smem(L, ns) <= kSrceDynMax) return ns;
   return 1;
 }
 /// One point per CTA until every SM has its CTAs, then more: a launch lasts as long as its longest
@@ -406,7 +409,7 @@ void srce_set_ctas_per_sm(const pt::SrceLayout& L, int ctas) {
 
 size_t srce_smem_bytes(const pt::SrceLayout& L) {
   const size_t b = srce_smem(L, 1);
-  return b + kSrceStatic <= 227 * 1024 ? b : 0;
+  return b <= kSrceDynMax ? b : 0;
 }
 
 void launch_sds4(const St4Dev* d, const st4::Params& hp, int npts, const float* a, const float* k,
