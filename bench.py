@@ -87,7 +87,7 @@ def parse():
     p.add_argument("--e2e-steps", type=int, default=None)
     p.add_argument("--no-cpu-baseline", action="store_true")
     p.add_argument("--no-autotune", action="store_true",
-                   help="skip the autotuner (DIA kernel, W3SRCE CTAs per SM) before timing")
+                   help="skip the autotuner (DIA kernel; W3SRCE's time on a sample) before timing")
     p.add_argument("--train-steps", type=int, default=30000,
                    help="surrogate workload: AdamW steps of batch 8192 before the timing")
     p.add_argument("--sur-lr", type=float, default=1e-3)
@@ -521,7 +521,7 @@ def run_b200_srce(args, quiet=False, npts=None, steps=None, warmup=None, igrid=1
     warmup = warmup or args.warmup
     st, t, sr, cfg, sig, pts = srce_inputs(synth, npts, 2026 + rank)
     grid = pkg.SrceGrid(igrid, t["rpar"], st["ipar"], synth.st4_registrations(st, t), cfg, sig, sr)
-    if not args.no_autotune:  # W3SRCE's CTAs per SM, timed on a sample of these points
+    if not args.no_autotune:  # W3SRCE timed on a sample of these points
         pkg.srce_autotune(igrid, pts)
     dev = torch.device("cuda", local)
     d0 = {k: torch.from_numpy(pts[k]).to(dev) for k in SRCE_ARRAYS}
@@ -1053,7 +1053,7 @@ def run_b200_multigrid(args):
 
     together = lambda: pkg.steps_run(igs, 1, handle)  # noqa: E731
 
-    if not args.no_autotune:  # W3SRCE's CTAs per SM on the first grid's points (one layout)
+    if not args.no_autotune:  # W3SRCE timed on the first grid's points
         pkg.srce_autotune(grids[0]["ig"], grids[0]["inputs"][2])
     # The grids' graphs one after another (the unfused form), from the initial state.
     record_all()

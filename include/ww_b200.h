@@ -149,11 +149,10 @@ int ww_snl1_autotune(int igrid);
  * faults, hangs or stays in flight, and the next call with bytes = 0 runs normally. */
 int ww_snl1_test_stall(int igrid, int bytes);
 
-/* B200 extension (the autotuner). The W3SRCE kernels' CTAs per SM, each count with the
- * shared-memory carveout that fits it (the rest of the SM's memory is L1), timed on a sample
- * of the caller's own points (arguments as ww_srce_batch takes them, host arrays, read only:
- * the sample runs on device copies): the fastest is kept for every later W3SRCE launch in the
- * process. Synchronous. Returns the CTAs per SM chosen, or -1. */
+/* B200 extension (the autotuner). The W3SRCE kernels are built for one CTA per SM, so there is
+ * nothing to choose: the call times W3SRCE on a sample of the caller's own points (arguments as
+ * ww_srce_batch takes them, host arrays, read only: the sample runs on device copies) and records
+ * the time for ww_autotune_report. Synchronous. Returns the CTAs per SM (1), or -1. */
 int ww_srce_autotune(int igrid, int it, int inflags24, int flogrd57, int flogrd58, float dtg,
                      int npts, const float* spec, const float* wn1, const float* cg1,
                      const float* pin, const float* psc, const float* whitecap,

@@ -378,11 +378,9 @@ int ww_srce_autotune(int igrid, int it, int inflags24, int flogrd57, int flogrd5
     SrceDev host{};
     if (!prepare(igrid, *g, host, "ww_srce_autotune")) return -1;
     const pt::SrceLayout& L = host.L;
-    const int maxc = srce_max_ctas_per_sm(L);
-    // A sample of the caller's points, four times the most CTAs that can be resident, so every
-    // candidate runs several points per CTA (the queue's tail is a small part of the time).
-    const int sms = runtime().sm_count;
-    const int n = std::min(npts, 4 * maxc * sms);
+    // A sample of the caller's points that fills every slot four times, so the queue's tail is a small
+    // part of the time.
+    const int n = std::min(npts, 4 * kSrceMinBlocks * pt::kSlots * runtime().sm_count);
     const size_t ns = static_cast<size_t>(n) * L.nspec, nk = static_cast<size_t>(n) * L.nk;
     struct Buf {
       float* p = nullptr;
@@ -402,8 +400,6 @@ int ww_srce_autotune(int igrid, int it, int inflags24, int flogrd57, int flogrd5
     up(s0.p, spec, ns), up(w.p, wn1, nk), up(c.p, cg1, nk), up(pn.p, pin, n * static_cast<size_t>(srce::NPIN));
     up(q0.p, psc, n * static_cast<size_t>(srce::NPSC)), up(wc0.p, whitecap, 4 * static_cast<size_t>(n));
     up(tb0.p, taubbl, 2 * static_cast<size_t>(n)), up(ti0.p, tauice, 2 * static_cast<size_t>(n));
-    std::vector<int> cands;
-    for (int k = maxc; k >= 1; --k) cands.push_back(k);
     cudaStream_t st = runtime().stream;
     const SrceStep step{it, inflags24, flogrd57, flogrd58, dtg};
     auto d2d = [&](float* d, const float* s_, size_t k, cudaStream_t ss) {
@@ -412,17 +408,13 @@ int ww_srce_autotune(int igrid, int it, int inflags24, int flogrd57, int flogrd5
     const std::string key = "srce ctas/SM " + std::to_string(L.nk) + "x" + std::to_string(L.nth) +
                             " " + tune::device_key();
     const int best = tune::pick(
-        key, cands,
-        [&](int ctas, cudaStream_t ss) {
+        key, {kSrceMinBlocks},
+        [&](int, cudaStream_t ss) {
           launch_srce(host, step, n, s1.p, nullptr, w.p, c.p, pn.p, q1.p, wc1.p, tb1.p, ti1.p,
                       reinterpret_cast<int*>(sh.p), g->work, ss);
-          (void)ctas;
         },
-        [&](int ctas, cudaStream_t ss) {
-          // the candidate's CTAs and carveout, and the sample's inputs restored (W3SRCE updates
-          // them in place)
-          WWB_CHECK(cudaStreamSynchronize(ss));
-          srce_set_ctas_per_sm(L, ctas);
+        [&](int, cudaStream_t ss) {
+          // the sample's inputs restored (W3SRCE updates them in place)
           srce_reserve(L, n, g->work, ss);
           d2d(s1.p, s0.p, ns, ss), d2d(q1.p, q0.p, n * static_cast<size_t>(srce::NPSC), ss);
           d2d(wc1.p, wc0.p, 4 * static_cast<size_t>(n), ss);
@@ -431,7 +423,6 @@ int ww_srce_autotune(int igrid, int it, int inflags24, int flogrd57, int flogrd5
         },
         st, 2);
     WWB_CHECK(cudaStreamSynchronize(st));
-    srce_set_ctas_per_sm(L, best == maxc ? 0 : best);
     g_status.ok();
     return best;
   } catch (const std::exception& e) {

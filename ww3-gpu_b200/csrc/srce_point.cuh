@@ -100,7 +100,7 @@ struct SrceLayout {
   int tslot;           ///< transient floats a slot needs outside the DIA
   int dia;             ///< transient floats of one slot's DIA
   // global scratch per slot
-  int specinit, vdin, vsnl, vdnl, vsds, vdds, vsdb, da, alen, work0, work1;
+  int specinit, vdin, vsnl, vdnl, vsds, vdds, vsdb, da, alen;
   int total_s;         ///< floats of shared memory with one slot
   int total_g;         ///< floats of global scratch per slot
 };
@@ -169,8 +169,6 @@ inline SrceLayout srce_layout(const st4::Params& q, const Snl1Dev& n) {
   L.vsdb = g; g += R;
   // The DIA's DA1P DA1M DA2P DA2M and DA1C + DA2C; W3SDS4's two bin arrays (SSDSC(1) = 2, 3).
   L.da = g;
-  L.work0 = g;
-  L.work1 = g + R;
   const int d = 4 * r4(L.alen) + R;
   g += d > 2 * R ? d : 2 * R;
   L.total_g = (g + 31) & ~31;
@@ -900,7 +898,6 @@ template <class G>
 WWB_PD void scan_serial(const Grp& c, const G& x, const SlotList& l, const Sin4At& at) {
   const SrceLayout& L = *x.L;
   const st4::Params& p = *x.q;
-  const Fields& f = *x.f;
   const int nk = L.nk, nth = x.nth(), T4 = (nth + 3) & ~3;
   const bool plain = scan_plain(p);
   constexpr int kPerWarp = Grp::kLanes / kScanLanes;
@@ -1027,7 +1024,7 @@ WWB_UNROLL(1)
 /// by the same 50 phase speeds in every substep, and this is a third of a division's latency.
 WWB_PD float div_by(float a, float b, float y) {
   const float m = fabs_f(a);
-  if (!((m >= 0x1p-80f && m <= 0x1p80f || a == 0.0f) && y != 0.0f)) return a / b;
+  if (!(((m >= 0x1p-80f && m <= 0x1p80f) || a == 0.0f) && y != 0.0f)) return a / b;
   float q = a * y;
   q = dm::fma_f(dm::fma_f(-b, q, a), y, q);
   return dm::fma_f(dm::fma_f(-b, q, a), y, q);

@@ -106,13 +106,6 @@ struct SrceRecorded {
   pt::SrceLayout L;
 };
 
-/// CTAs per SM of the W3SRCE kernels when every one that fits is resident.
-int srce_max_ctas_per_sm(const pt::SrceLayout& L);
-
-/// Limits the W3SRCE kernels to `ctas` CTAs per SM (0: all that fit) with the shared-memory
-/// carveout they need, the rest of the SM's memory left to L1 (the autotuner's choice).
-void srce_set_ctas_per_sm(const pt::SrceLayout& L, int ctas);
-
 /// Allocates launch_srce_multi's work buffers for `total` points of layout L (synchronous).
 void srce_multi_reserve(const pt::SrceLayout& L, int total, SrceWork& work);
 

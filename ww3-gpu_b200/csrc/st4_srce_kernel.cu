@@ -292,11 +292,10 @@ OneKernel one_kernel(const pt::SrceLayout& L) {
   return L.nth == 36 ? srce_kernel<36> : L.nth == 24 ? srce_kernel<24> : srce_kernel<0>;
 }
 MultiKernel multi_kernel(int nth) {
+  // No form for 24: eight grids of 25 x 24 bins, 3,924 points, a step 10.4-12.6 ms with the general one
+  // and 10.3-12.2 with one of its own.
   return nth == 36 ? srce_multi_kernel<36> : srce_multi_kernel<0>;
 }
-
-/// CTAs per SM of the W3SRCE kernel (0: all that fit), set by the autotuner.
-int g_srce_ctas_per_sm = 0;
 
 /// Resident CTAs of an ST4 kernel at this shared memory, at most one per point.
 template <class K>
@@ -326,36 +325,28 @@ struct SrcePlan {
   int ns, grid;
   size_t smem;
 };
-int srce_per_sm(const pt::SrceLayout& L, int ns, bool multi = false) {
-  const size_t smem = srce_smem(L, ns);
-  const void* const k = multi ? reinterpret_cast<const void*>(multi_kernel(L.nth))
-                              : reinterpret_cast<const void*>(one_kernel(L));
-  WWB_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kSrceDynMax)));
-  int per_sm = 0;
-  WWB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kSrceBlock, smem));
-  if (per_sm < 1) throw CudaError(cudaErrorInvalidConfiguration, "srce occupancy");
-  return g_srce_ctas_per_sm > 0 && g_srce_ctas_per_sm < per_sm ? g_srce_ctas_per_sm : per_sm;
-}
-/// Slots a CTA of this layout can have: all of them where as many CTAs fit an SM as with one.
+/// Slots a CTA of this layout can have.
 int srce_max_slots(const pt::SrceLayout& L) {
   for (int ns = pt::kSlots; ns > 1; --ns)
     if (srce_smem(L, ns) <= kSrceDynMax) return ns;
   return 1;
 }
-/// One point per CTA until every SM has its CTAs, then more: a launch lasts as long as its longest
-/// point, and a point alone in its CTA is integrated fastest.
-SrcePlan srce_plan(const pt::SrceLayout& L, int npts, bool multi = false) {
+/// The fewest slots with which the points fit the SMs' CTAs at once, and as many CTAs as that fills: a
+/// launch lasts as long as its longest point, and a point is integrated faster the fewer share its CTA
+/// (149 points on 148 SMs run as 75 CTAs of two). CTAs per SM are the one that the kernels are built for.
+SrcePlan srce_plan(const pt::SrceLayout& L, int npts) {
   if (srce_smem_bytes(L) == 0)
     throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
-  const int most = srce_max_slots(L), sms = runtime().sm_count;
-  for (int ns = 1;; ++ns) {
-    const long long ctas = static_cast<long long>(srce_per_sm(L, ns, multi)) * sms;
-    if (ns == most || ctas * ns >= npts) {
-      const long long want = (static_cast<long long>(npts) + ns - 1) / ns;
-      return SrcePlan{ns, static_cast<int>(want < ctas ? want : ctas), srce_smem(L, ns)};
-    }
-  }
+  const int most = srce_max_slots(L);
+  const long long ctas = static_cast<long long>(kSrceMinBlocks) * runtime().sm_count;
+  int ns = 1;
+  while (ns < most && ctas * ns < npts) ++ns;
+  const long long want = (static_cast<long long>(npts) + ns - 1) / ns;
+  return SrcePlan{ns, static_cast<int>(want < ctas ? want : ctas), srce_smem(L, ns)};
+}
+void srce_allow(const void* k) {
+  WWB_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kSrceDynMax)));
 }
 void srce_reserve_plan(const pt::SrceLayout& L, const SrcePlan& plan, SrceWork& work) {
   const size_t need = static_cast<size_t>(plan.grid) * plan.ns * static_cast<size_t>(L.total_g);
@@ -368,44 +359,18 @@ void srce_reserve_plan(const pt::SrceLayout& L, const SrcePlan& plan, SrceWork& 
     work.scratch_n = need;
   }
 }
-void set_carveout(const pt::SrceLayout& L, int pct) {
-  WWB_CHECK(cudaFuncSetAttribute(reinterpret_cast<const void*>(one_kernel(L)),
-                                 cudaFuncAttributePreferredSharedMemoryCarveout, pct));
-  WWB_CHECK(cudaFuncSetAttribute(reinterpret_cast<const void*>(multi_kernel(L.nth)),
-                                 cudaFuncAttributePreferredSharedMemoryCarveout, pct));
-}
+/// Whether the work buffers are large enough for the plan.
 bool srce_reserved(const pt::SrceLayout& L, const SrcePlan& plan, const SrceWork& work) {
   return work.counter != nullptr && static_cast<size_t>(plan.grid) * plan.ns *
                                             static_cast<size_t>(L.total_g) <= work.scratch_n;
 }
+void srce_reserve(const pt::SrceLayout& L, const SrcePlan& plan, SrceWork& work, cudaStream_t st) {
+  if (srce_reserved(L, plan, work)) return;
+  WWB_CHECK(cudaStreamSynchronize(st));  // earlier launches may still use the old buffers
+  srce_reserve_plan(L, plan, work);
+}
 
 }  // namespace
-
-int srce_max_ctas_per_sm(const pt::SrceLayout& L) {
-  if (srce_smem_bytes(L) == 0)
-    throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
-  const int keep = g_srce_ctas_per_sm;
-  g_srce_ctas_per_sm = 0;
-  set_carveout(L, cudaSharedmemCarveoutDefault);
-  const int all = srce_per_sm(L, srce_max_slots(L));
-  srce_set_ctas_per_sm(L, keep);  // the carveout of the current choice again
-  return all;
-}
-
-void srce_set_ctas_per_sm(const pt::SrceLayout& L, int ctas) {
-  if (srce_smem_bytes(L) == 0)
-    throw CudaError(cudaErrorInvalidConfiguration, "W3SRCE working set too large");
-  g_srce_ctas_per_sm = ctas > 0 ? ctas : 0;
-  // The shared-memory carveout just large enough for that many CTAs (their dynamic and static
-  // shared memory and the 1 KiB the system keeps per CTA): the rest of the SM's 256 KiB is L1.
-  int pct = cudaSharedmemCarveoutDefault;
-  if (ctas > 0) {
-    const size_t per_cta = srce_smem(L, srce_max_slots(L)) + kSrceStatic + 1024;
-    pct = static_cast<int>((100 * ctas * per_cta + 228 * 1024 - 1) / (228 * 1024));
-    if (pct > 100) pct = 100;
-  }
-  set_carveout(L, pct);
-}
 
 size_t srce_smem_bytes(const pt::SrceLayout& L) {
   const size_t b = srce_smem(L, 1);
@@ -454,22 +419,20 @@ void launch_spr4(const St4Dev* d, const st4::Params& hp, int npts, const float* 
 
 void srce_reserve(const pt::SrceLayout& L, int npts, SrceWork& work, cudaStream_t st) {
   if (npts <= 0) return;
-  const SrcePlan plan = srce_plan(L, npts);
-  if (srce_reserved(L, plan, work)) return;
-  WWB_CHECK(cudaStreamSynchronize(st));  // earlier launches may still use the old buffers
-  srce_reserve_plan(L, plan, work);
+  srce_reserve(L, srce_plan(L, npts), work, st);
 }
 
 void srce_multi_reserve(const pt::SrceLayout& L, int total, SrceWork& work) {
-  srce_reserve_plan(L, srce_plan(L, total > 0 ? total : 1, true), work);
+  srce_reserve_plan(L, srce_plan(L, total > 0 ? total : 1), work);
 }
 
 void launch_srce_multi(const SrceJob* jobs_dev, int njobs, int total, const pt::SrceLayout& L,
                        SrceWork& work, cudaStream_t st) {
   if (total <= 0) return;
-  const SrcePlan plan = srce_plan(L, total, true);
+  const SrcePlan plan = srce_plan(L, total);
   if (!srce_reserved(L, plan, work))
     throw CudaError(cudaErrorInvalidValue, "launch_srce_multi: work buffers not reserved");
+  srce_allow(reinterpret_cast<const void*>(multi_kernel(L.nth)));
   WWB_CHECK(cudaMemsetAsync(work.counter, 0, sizeof(int), st));
   multi_kernel(L.nth)<<<plan.grid, kSrceBlock, plan.smem, st>>>(jobs_dev, njobs, total, plan.ns,
                                                                 work.counter, work.scratch);
@@ -484,7 +447,8 @@ void launch_srce(const SrceDev& dev, SrceStep step, int npts, float* spec, const
   const SrcePlan plan = srce_plan(L, npts);
   // The work buffers fit after srce_reserve; otherwise (re)allocate them first, after the
   // previous launches on this stream that may still read the old ones.
-  srce_reserve(L, npts, work, st);
+  srce_reserve(L, plan, work, st);
+  srce_allow(reinterpret_cast<const void*>(one_kernel(L)));
   WWB_CHECK(cudaMemsetAsync(work.counter, 0, sizeof(int), st));
   const SrceJob job{nullptr, step, npts,     0,      spec,   jsea, wn1, cg1,
                     pin,     psc,  whitecap, taubbl, tauice, shave};
