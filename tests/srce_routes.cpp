@@ -29,6 +29,52 @@ int routes_layout(unsigned char* out, int cap) {
   return static_cast<int>(sizeof L);
 }
 
+/// W3SIN4, W3SDS4 and W3SPR4 as W3SRCE's phases form them, for one point in one slot: spec (NSPEC), wn1 and
+/// cg1 (NK), the point's packet pin, what W3SPR4 left (ustar, usdir, dlwmean, z0) and the stress entering
+/// W3SPR4. Out: D, LLWS, tau[4] = TAUWX TAUWY TAUWNX TAUWNY; SRHS, DDIAG, BRLAMBDA, WHITECAP; W3SPR4's 12.
+void routes_terms(const float* spec, const float* wn1, const float* cg1, const float* pin, float ustar,
+                  float usdir, float dlwmean, float z0, float tauwx, float tauwy, const int* llws_in,
+                  float* d, int* llws, float* tau, float* srhs, float* ddiag, float* brlambda,
+                  float* whitecap, float* spr4) {
+  const pt::SrceLayout L = pt::srce_layout(g_p, g_ndev);
+  std::vector<float> w(L.total_s + 4), gw(L.total_g + 4);
+  static pt::SrceSh sh;
+  sh = pt::SrceSh{};
+  const pt::Grp c{0, 1};
+  const pt::SrceGroup<0> x{&g_sp, &g_sgrid, &g_p, &g_fields, &g_ndev, &L, w.data(), gw.data(),
+                           w.data() + L.common + L.ws, &sh, 1, nullptr};
+  std::memcpy(x.s(0, L.spec), spec, sizeof(float) * L.nspec);
+  std::memcpy(x.s(0, L.wn1), wn1, sizeof(float) * L.nk);
+  std::memcpy(x.s(0, L.cg1), cg1, sizeof(float) * L.nk);
+  pt::SlotList l{};
+  l.add(0);
+  sh.in = pt::srce_in(1, 0, 1, 1, 900.0f, pin);
+  pt::srce_common(c, x);
+  pt::srce_begin(c, x, l);
+  sh.r.ustar = ustar;
+  sh.r.usdir = usdir;
+  sh.r.dlwmean = dlwmean;
+  sh.r.z0 = z0;
+  pt::srce_sin4(c, x, l);
+  std::memcpy(d, x.gs(0, L.vdin), sizeof(float) * L.nspec);
+  for (int i = 0; i < L.nspec; ++i) llws[i] = x.llws(0)[i];
+  const float t[4] = {sh.tauwx, sh.tauwy, sh.tauwax, sh.tauway};
+  std::memcpy(tau, t, sizeof t);
+  pt::srce_sds4(c, x, l);
+  std::memcpy(srhs, x.gs(0, L.vsds), sizeof(float) * L.nspec);
+  std::memcpy(ddiag, x.gs(0, L.vdds), sizeof(float) * L.nspec);
+  std::memcpy(brlambda, x.tr(0), sizeof(float) * L.nspec);
+  std::memcpy(whitecap, sh.whitecap, sizeof sh.whitecap);
+  for (int i = 0; i < L.nspec; ++i) x.llws(0)[i] = static_cast<unsigned char>(llws_in[i]);
+  sh.tauwx = tauwx;
+  sh.tauwy = tauwy;
+  pt::spr4_sums(c, x, l, 0);
+  pt::spr4_chains(c, x, l, 0);
+  sh.r.dlwmean = dm::atan2f(sh.chains[1], sh.chains[0]);
+  sh.r.amax = sh.chains[2];
+  std::memcpy(spr4, &sh.r, sizeof sh.r);
+}
+
 /// Mismatches over n seeded arguments of: 0 div_core (reciprocal seed an ulp off either way), 1 expf_q /
 /// expf_neg, 2 logf_q, 3 powf_core / powf_mid, 4 sincosf_core, 5 atan2f_core, 6 div_by.
 void routes_libm(long n, unsigned long long seed, long* bad) {

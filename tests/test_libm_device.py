@@ -38,3 +38,18 @@ def test_device_libm_equals_glibc(checker, fn, stride):
     assert m, out
     assert int(m.group(1)) == (1 << 32) // stride
     assert int(m.group(2)) == 0, out
+
+
+def test_branch_free_forms_equal_general(tmp_path):
+    """The forms that W3SRCE's kernels use instead of the general functions, with the device's reciprocal
+    seed (tests/libm_forms_check.cu)."""
+    exe = tmp_path / "libm_forms_check"
+    subprocess.run(["/usr/local/cuda/bin/nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3",
+                    "-std=c++17", "-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false",
+                    "-Xcompiler", "-ffp-contract=off", "-ccbin", "/usr/bin/g++",
+                    str(ROOT / "tests" / "libm_forms_check.cu"), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+    rows = [line.split() for line in out.splitlines()]
+    assert len(rows) == 9
+    for name, seen, bad in rows:
+        assert int(seen) > 1 << 27 and int(bad) == 0, out
