@@ -260,7 +260,7 @@ struct SlotList {
 };
 static_assert(kSlots <= 8, "SlotList holds eight 4-bit numbers");
 /// Slots that W3SDS4's sums over tables take together, so that a table row is read once for all of them
-/// (9,520 points: two 101 ms, four 98.7, eight 98; 777 points with Romero's breaking: 18.2, 18.5, 19.1).
+/// (9,520 points: two 106.7 ms, four 102.3, eight 106.8; 777 points with Romero's breaking: 19.1, 19.2, 20.4).
 constexpr int kTogether = 4;
 
 /// What the working warps leave for the tail warp.
@@ -1021,7 +1021,8 @@ WWB_UNROLL(1)
 /// a / b for b in [2^-20, 2^20], correctly rounded, from y = 1 / b correctly rounded (0: unknown): two steps q + (a - b q) y with fused
 /// multiply-adds (Markstein 1990, IBM J. Res. Dev. 34: one step from a quotient within an ulp is exact,
 /// the first makes it so), where nothing under- or overflows; else the division itself. The tail divides
-/// by the same 50 phase speeds in every substep, and this is a third of a division's latency.
+/// by the same 50 phase speeds in every substep, and this is a third of a division's latency. a = -0 gives
+/// +0, which changes no result there.
 WWB_PD float div_by(float a, float b, float y) {
   const float m = fabs_f(a);
   if (!(((m >= 0x1p-80f && m <= 0x1p80f) || a == 0.0f) && y != 0.0f)) return a / b;
